@@ -122,7 +122,7 @@ int run_partition(cfg_ctx* c, std::vector<uint32_t>& inst_h, std::vector<uint32_
         a.packed = c->d_packed; a.frag_off = c->d_frag_off; a.frag_len = c->d_frag_len;
         a.n_frags = c->n_frags; a.n_bases = c->n_bases;
         a.k = c->p.k; a.l = c->p.l; a.w = c->p.k - c->p.l;
-        a.gmask = G - 1; a.seed0 = wy_seed0_host(); a.seg = 2048;
+        a.gmask = G - 1; a.seed0 = wy_seed0_host(); a.seg = partition_segment(c->n_bases, a.w);
         a.recs = c->flat.as<uint64_t>(); a.rec_cap = cap;
         a.rec_cursor = &c->misc.as<MiscWords>()->rec_cursor;
         a.hist = nullptr;   // the bucket sort counts records and instances per subgraph

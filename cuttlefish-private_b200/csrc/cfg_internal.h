@@ -68,6 +68,18 @@ struct PartitionArgs {
     // l-mer's reverse complement is computed from the l-mer itself
     const uint64_t* rcw;
 };
+// Stream bases per warp of a partition launch.  A warp walks its segment 32 bases at a
+// time, one chunk after another, and pays about three more chunks to prime the window
+// before the segment and to finish the last run past it (more for a wide window), so long
+// segments waste the least -- but a job cut into fewer than about 8192 of them leaves SMs
+// idle (148 SMs hold 3552 warps of this kernel).  Measured, k = 31, l = 20, by bases per
+// segment: 50 kbp 2048 -> 69 us, 512 -> 28, 128 -> 17; 5 Mbp 2048 -> 115 us, 1024 -> 97,
+// 512 -> 93, 256 -> 99, 128 -> 118; 24 Mbp 2048 -> 337 us, 1024 -> 345, 512 -> 371.
+inline uint32_t partition_segment(uint64_t n_bases, uint32_t w) {
+    const uint64_t even = (n_bases / 8192 + 31) & ~31ull, least = (4 * w > 128 ? 4 * w + 31 : 128) & ~31u;
+    return (uint32_t)(even < least ? least : even < 2048 ? even : 2048);
+}
+
 // rcw[w] for the packed words [w0, w1): the reverse complement of word w.
 void launch_rc_words(const uint64_t* packed, uint64_t w0, uint64_t w1, uint64_t* rcw, cudaStream_t s);
 

@@ -125,7 +125,7 @@ extern "C" int cfg_partition_noalloc(int device, const cfg_params* p, const uint
         a.k = p->k; a.l = p->l; a.w = p->k - p->l;
         a.gmask = p->graph_count - 1;
         a.seed0 = wy_seed0_host();
-        a.seg = 2048;
+        a.seg = partition_segment(n_bases, a.w);
         a.recs = (uint64_t*)(s + OFF_RECS); a.rec_cap = NOALLOC_MAX_RECORDS;
         a.rec_cursor = &((NoallocMisc*)(s + OFF_MISC))->rec_cursor;
         a.hist = (unsigned long long*)(s + OFF_HIST);
