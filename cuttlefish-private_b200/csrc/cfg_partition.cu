@@ -274,34 +274,7 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32) k_partition(const Partit
     stage_flush(a, st);
 }
 
-// Exclusive scan of the per-subgraph record counts (one block).
-__global__ void __launch_bounds__(1024) k_bucket_scan(const unsigned long long* __restrict__ hist, uint32_t G,
-                                                      uint32_t* bucket_off, uint32_t* inst, uint32_t* fill) {
-    __shared__ uint32_t part[1024];
-    const uint32_t t = threadIdx.x;
-    const uint32_t per = (G + 1023) / 1024;
-    const uint32_t b0 = t * per, b1 = min(b0 + per, G);
-    uint32_t sum = 0;
-    for (uint32_t b = b0; b < b1; ++b) sum += (uint32_t)hist[b];
-    part[t] = sum;
-    __syncthreads();
-    for (uint32_t d = 1; d < 1024; d <<= 1) {
-        const uint32_t v = t >= d ? part[t - d] : 0;
-        __syncthreads();
-        part[t] += v;
-        __syncthreads();
-    }
-    uint32_t run = part[t] - sum;
-    for (uint32_t b = b0; b < b1; ++b) {
-        bucket_off[b] = run;
-        run += (uint32_t)hist[b];
-        inst[b] = (uint32_t)(hist[b] >> 32);
-        fill[b] = 0;
-    }
-    if (t == 1023) bucket_off[G] = part[1023];
-}
-
-// Multi-block scan for batches (millions of buckets): 8192 entries per block.
+// Multi-block scans take 8192 entries per block.
 constexpr uint32_t SCAN_PER_THREAD = 8, SCAN_BLOCK = 1024, SCAN_CHUNK = SCAN_PER_THREAD * SCAN_BLOCK;
 
 __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* warp_sums, uint32_t& total) {
@@ -328,6 +301,47 @@ __device__ __forceinline__ uint32_t block_excl_scan(uint32_t v, uint32_t* warp_s
     return before + x - v;
 }
 
+// Exclusive scan of the per-subgraph record counts by one block, 8192 entries at a time: a
+// thread's 8 entries are 64 consecutive bytes (whole sectors), read with 16-byte loads and
+// kept in registers between the sum and the write, so the histogram is read once.  Latency
+// bound: 16384 subgraphs take 6 us where one pass of 16 strided entries a thread, a
+// ten-barrier scan and a second read of the histogram took 44 us.
+__global__ void __launch_bounds__(SCAN_BLOCK) k_bucket_scan(const unsigned long long* __restrict__ hist, uint32_t G,
+                                                            uint32_t* bucket_off, uint32_t* inst, uint32_t* fill) {
+    __shared__ uint32_t ws[32];
+    uint32_t run0 = 0;
+    for (uint32_t t0 = 0; t0 < G; t0 += SCAN_CHUNK) {
+        const uint32_t b0 = t0 + threadIdx.x * SCAN_PER_THREAD;
+        unsigned long long h[SCAN_PER_THREAD];
+        const bool whole = b0 + SCAN_PER_THREAD <= G;
+#pragma unroll
+        for (uint32_t i = 0; i < SCAN_PER_THREAD; i += 2) {
+            if (whole) {
+                const ulonglong2 v = *(const ulonglong2*)(hist + b0 + i);
+                h[i] = v.x; h[i + 1] = v.y;
+            } else {
+                h[i] = b0 + i < G ? hist[b0 + i] : 0ull;
+                h[i + 1] = b0 + i + 1 < G ? hist[b0 + i + 1] : 0ull;
+            }
+        }
+        uint32_t sum = 0, total;
+#pragma unroll
+        for (uint32_t i = 0; i < SCAN_PER_THREAD; ++i) sum += (uint32_t)h[i];
+        uint32_t run = run0 + block_excl_scan(sum, ws, total);
+#pragma unroll
+        for (uint32_t i = 0; i < SCAN_PER_THREAD; ++i) {
+            if (b0 + i >= G) break;
+            bucket_off[b0 + i] = run;
+            inst[b0 + i] = (uint32_t)(h[i] >> 32);
+            fill[b0 + i] = 0;
+            run += (uint32_t)h[i];
+        }
+        run0 += total;
+    }
+    if (threadIdx.x == 0) bucket_off[G] = run0;
+}
+
+// Multi-block scan for batches (millions of buckets).
 __global__ void __launch_bounds__(SCAN_BLOCK) k_scan_reduce(const unsigned long long* __restrict__ hist, uint32_t n,
                                                             uint32_t* partials) {
     __shared__ uint32_t ws[32];
@@ -423,7 +437,7 @@ void launch_rc_words(const uint64_t* packed, uint64_t w0, uint64_t w1, uint64_t*
 
 void launch_bucket_scan(const unsigned long long* hist, uint32_t G, uint32_t* bucket_off, uint32_t* inst,
                         uint32_t* fill, cudaStream_t s) {
-    k_bucket_scan<<<1, 1024, 0, s>>>(hist, G, bucket_off, inst, fill);
+    k_bucket_scan<<<1, SCAN_BLOCK, 0, s>>>(hist, G, bucket_off, inst, fill);
 }
 
 void launch_bucket_scan_large(const unsigned long long* hist, uint32_t n, uint32_t* bucket_off, uint32_t* inst,
