@@ -185,7 +185,7 @@ int run_partition(cfg_ctx* c, std::vector<uint32_t>& inst_h, std::vector<uint32_
 
 // One launch: subgraphs sharing a table shape.  cluster 0 = global arena tables
 // (per-entry offset/capacity), else `cluster` CTAs with `per` slots each.
-struct Launch { std::vector<uint32_t> list; std::vector<uint64_t> off; std::vector<uint32_t> cap; uint32_t per = 0; uint32_t cluster = 0; };
+struct Launch { std::vector<uint32_t> list; std::vector<uint64_t> off; std::vector<uint32_t> cap; uint32_t per = 0; uint32_t cluster = 0; uint32_t threads = 0; };
 
 int launch_plan(cfg_ctx* c, const std::vector<Launch>& plan, uint64_t arena_slots) {
     const int W = c->words;
@@ -219,14 +219,13 @@ int launch_plan(cfg_ctx* c, const std::vector<Launch>& plan, uint64_t arena_slot
         a.dump = (c->p.flags & CFG_FLAG_DUMP_STATES) ? c->dump.as<StateOut>() : nullptr; a.dump_cap = c->dump_cap;
         a.retry = c->retry.as<uint32_t>(); a.cnt = c->counters.as<Counters>();
         a.err = &c->misc.as<MiscWords>()->err;
-        // a quarter of the slots, up to the table class's largest CTA (k <= 31: 512 threads,
-        // two CTAs per SM, and 1024 for the 8192-slot tables; k > 32: 256 up to 2048 slots,
-        // three CTAs per SM); arena tables: that largest CTA
-        const uint32_t tmax = subgraph_max_threads(W, L.cluster == 0 ? 0u : L.per);
-        const uint32_t div = c->p.slots_per_thread ? c->p.slots_per_thread : 4;
+        // the table shape's threads, unless the caller set slots per thread; clusters and arena
+        // tables: a quarter of the slots, or the largest CTA
+        const uint32_t tmax = subgraph_max_threads(W, L.cluster == 0 ? 0u : L.per), div = c->p.slots_per_thread;
         const uint32_t threads = L.cluster == 0 ? tmax
+                                 : L.cluster == 1 && !div ? L.threads
                                  : L.cluster == 1 && L.per > 4096 ? tmax
-                                 : std::min<uint32_t>(tmax, (std::max<uint32_t>(64, L.per / div) + 31) / 32 * 32);
+                                 : std::min<uint32_t>(tmax, (std::max<uint32_t>(64, L.per / (div ? div : 4)) + 31) / 32 * 32);
         CK(launch_subgraphs(a, W, L.cluster, threads, c->stream));
         c->launches += 1;
         at += L.list.size();
@@ -262,7 +261,8 @@ int run_subgraphs(cfg_ctx* c, const std::vector<uint32_t>& inst_h) {
     // expected distinct vertices per k-mer instance, in percent; tables are sized for
     // a load factor near one half of that estimate
     const uint32_t load = c->p.table_load_pct ? c->p.table_load_pct : 100;
-    const uint32_t per_max = subgraph_max_per_cta(W);   // one CTA's table
+    uint32_t n_shapes = 0;
+    const LocalShape* shapes = local_shapes(W, n_shapes);   // one CTA's table
     const uint32_t per_cl = subgraph_cluster_per_cta(W);   // each CTA of a cluster
     // k <= 31: clusters of up to 8 CTAs beat arena tables in HBM; k > 32 (24-byte key and
     // state, 128-register kernels, one CTA per SM) the L2-resident arena tables win
@@ -302,14 +302,16 @@ int run_subgraphs(cfg_ctx* c, const std::vector<uint32_t>& inst_h) {
         bool overflow = false;
         for (int pass = 0; pass < 12 && !work.empty(); ++pass) {
             std::vector<Launch> plan;
-            int shape_at[9 * 32];
-            std::fill(shape_at, shape_at + 9 * 32, -1);
+            int shape_at[16 + 9];   // launch of each one-CTA shape, then of each cluster size
+            std::fill(shape_at, shape_at + 16 + 9, -1);
             Launch glob; glob.cluster = 0;
             uint64_t arena_slots = 0;
             for (uint32_t g : work) {
                 const uint64_t w = cur_want[g];
-                uint32_t cl, per;
-                if (w <= per_max) { cl = 1; per = next_pow2(w); }
+                uint32_t cl, per, sh = 0;
+                const uint64_t fit = local_fit(W, w);
+                while (sh < n_shapes && shapes[sh].slots < fit) ++sh;
+                if (sh < n_shapes) { cl = 1; per = shapes[sh].slots; }
                 else if (w <= (uint64_t)per_cl * max_cluster) { cl = (uint32_t)((w + per_cl - 1) / per_cl); per = per_cl; }
                 else {
                     const uint32_t cap = next_pow2(w);
@@ -317,11 +319,12 @@ int run_subgraphs(cfg_ctx* c, const std::vector<uint32_t>& inst_h) {
                     arena_slots += cap;
                     continue;
                 }
-                // launch of this shape: one per (cluster size, log2 slots)
-                const uint32_t sk = cl * 32 + (31 - __builtin_clz(per));
+                // one launch per shape
+                const uint32_t sk = cl == 1 ? sh : 16 + cl;
                 if (shape_at[sk] < 0) {
                     shape_at[sk] = (int)plan.size();
                     plan.emplace_back(); plan.back().per = per; plan.back().cluster = cl;
+                    plan.back().threads = cl == 1 ? shapes[sh].threads : 0;
                 }
                 plan[shape_at[sk]].list.push_back(g);
             }

@@ -219,7 +219,14 @@ int subgraph_occupancy(int words, uint32_t cluster, uint32_t threads, uint32_t p
 // bucket_off[0..n], inst[b], fill[b] = 0.  `partials` holds (n + 8191) / 8192 words.
 void launch_bucket_scan_large(const unsigned long long* hist, uint32_t n, uint32_t* bucket_off, uint32_t* inst,
                               uint32_t* fill, uint32_t* partials, cudaStream_t s);
-uint32_t subgraph_max_per_cta(int words);      // one CTA owning a whole table
+struct LocalShape { uint32_t slots, threads; };
+const LocalShape* local_shapes(int words, uint32_t& n);   // one-CTA tables of k-mers of `words` words, smallest first
+// Slots a one-CTA table must have for a subgraph that wants `want` (twice its expected
+// vertices).  k <= 31 keeps half load; wider k-mers take two thirds, for the extra CTA or
+// two per SM that the smaller table allows (500 Mbp, k = 63: 132 ms at half load, 110 at
+// 0.57, 98.5 at 0.67, 107 at 0.77; k = 127: 8.7 ms at half load, 7.3 at 0.62).
+inline uint64_t local_fit(int words, uint64_t want) { return words == 1 ? want : want * 3 / 4; }
+uint32_t subgraph_max_per_cta(int words);      // the largest of them
 // Largest CTA of a launch of `per`-slot tables (per 0: arena tables).
 uint32_t subgraph_max_threads(int words, uint32_t per);
 uint32_t subgraph_cluster_per_cta(int words);  // each CTA of a cluster

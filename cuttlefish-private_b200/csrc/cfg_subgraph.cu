@@ -1343,14 +1343,12 @@ __device__ __forceinline__ void carve(unsigned char* base, uint32_t per, unsigne
     wl = meta + per;
 }
 
-// One subgraph per CTA (per = the table's whole capacity) or per cluster.  LB: the
-// largest CTA.  k > 32 (104 registers at LB 512) has a second form for tables of up to
-// 2048 slots, LB 256 at three CTAs per SM (80 registers): a 512-thread CTA of the wide
-// form holds a whole SM's registers, so one subgraph's phase barriers idle the SM.
-// k > 63 runs 256-thread CTAs, two per SM (128 registers).
-constexpr int shared_min_blocks(int W, int LB) { return W > 2 ? 2 : LB <= 256 ? 3 : 1; }
+// One subgraph per CTA (per = the table's whole capacity) or per cluster.  LB bounds the
+// registers so that a full SM of CTAs of any table shape (local_shapes) holds LB threads:
+// 1024 at 64 registers for k <= 31, 768 at 80 for k <= 63, 512 at 128 beyond.
+constexpr int local_threads(int W) { return W == 1 ? 1024 : W == 2 ? 768 : 512; }
 template <int W, int MODE, int LB>
-__global__ void __launch_bounds__(LB, shared_min_blocks(W, LB)) k_subgraph_shared(const SubgraphArgs a) {
+__global__ void __launch_bounds__(LB, 1) k_subgraph_shared(const SubgraphArgs a) {
     extern __shared__ __align__(16) unsigned char smem[];
     __shared__ Block B;
     uint32_t rank = 0, nranks = 1;
@@ -1396,9 +1394,27 @@ __global__ void __launch_bounds__(GlobalBounds<W>::threads, GlobalBounds<W>::min
     }
 }
 
+// One-CTA table shapes, smallest first.  A subgraph's phases end in CTA-wide barriers and
+// its work comes in waves (paths are a seventh of the vertices), so a CTA waits much of the
+// time: what keeps an SM busy is several subgraphs at once.  `slots` is what lets c CTAs
+// share an SM's 228 KB (233472 / c - 2048 bytes of bookkeeping and reserve, over the slot's
+// bytes), `threads` the CTA's share of the SM's registers.  Tables in powers of two with a
+// thread per four slots (64 to 512) measured, subgraph kernels: 500 Mbp k = 63, 1000 k-mers
+// a subgraph (one 256-thread CTA of 2048 slots, three to an SM): 138.3 -> 98.5 ms here on
+// 1760 slots, four to an SM; 12 Mbp k = 127, 730 a subgraph: 13.6 -> 7.3 ms (the tail of
+// larger ones off the arena, three CTAs to an SM instead of two); 5 Mbp k = 31, 350 a
+// subgraph (1024 slots): 0.99 -> 0.76 ms with 128 threads instead of 256.  Finer k <= 31
+// shapes (720, 1536, 3152 slots) measured no better: longer probes for no more CTAs' worth
+// of latency hidden.
+constexpr LocalShape SHAPES_1[] = {{64, 64}, {128, 64}, {256, 64}, {520, 64}, {1128, 128}, {2344, 256}, {4096, 512}, {8192, 1024}};
+constexpr LocalShape SHAPES_2[] = {{64, 64}, {128, 64}, {256, 64}, {544, 64}, {1152, 128}, {1760, 160}, {2368, 256}, {3584, 384}, {7200, 768}};
+constexpr LocalShape SHAPES_4[] = {{64, 64}, {128, 64}, {256, 64}, {560, 64}, {1168, 128}, {1576, 160}, {2384, 256}, {4816, 512}};   // three or four key words
+
 // The kernels' shared-memory limit is always raised to the largest table any launch
 // uses (it is process-wide state: lowering it would break launches recorded in graphs).
-template <int W> constexpr size_t max_table_bytes() { return (size_t)(W == 1 ? 8192 : W == 2 ? 4096 : 2048) * slot_bytes(W); }
+template <int W> constexpr size_t max_table_bytes() {
+    return (size_t)(W == 1 ? 8192 : W == 2 ? 7200 : 4816) * slot_bytes(W);
+}
 template <typename K>
 cudaError_t raise_smem_limit(K kernel, size_t bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
@@ -1464,31 +1480,33 @@ __global__ void k_stripe_fixup(LmtigOut* lm, uint64_t lm_slice, const unsigned l
     }
 }
 
-uint32_t subgraph_max_per_cta(int words) { return words == 1 ? 8192 : words == 2 ? 4096 : 2048; }
+const LocalShape* local_shapes(int words, uint32_t& n) {
+    if (words == 1) { n = sizeof(SHAPES_1) / sizeof(LocalShape); return SHAPES_1; }
+    if (words == 2) { n = sizeof(SHAPES_2) / sizeof(LocalShape); return SHAPES_2; }
+    n = sizeof(SHAPES_4) / sizeof(LocalShape);
+    return SHAPES_4;
+}
+uint32_t subgraph_max_per_cta(int words) {
+    uint32_t n;
+    const LocalShape* sh = local_shapes(words, n);
+    return sh[n - 1].slots;
+}
 uint32_t subgraph_max_threads(int words, uint32_t per) {
-    if (words > 2) return 256;                            // k > 63: one 256-thread form
     if (per == 0) return words == 1 ? 512 : 256;          // arena tables
     if (words == 1) return per > 4096 ? 1024 : 512;
-    return per > 2048 ? 512 : 256;
+    if (words == 2) return per > 3584 ? 768 : per > 2368 ? 384 : 256;
+    return per > 2384 ? 512 : 256;
 }
 uint32_t subgraph_cluster_per_cta(int words) { return words == 1 ? 4096 : 2048; }
 
 namespace {
-// the kernel of a one-CTA shared-memory table, by key words and CTA size
+// the kernel of a one-CTA shared-memory table, by key words
 template <int W> cudaError_t launch_local_w(const SubgraphArgs& a, uint32_t threads, size_t bytes, cudaStream_t s,
                                             uint32_t grid, size_t limit) {
-    if constexpr (W == 1) return launch_shared(k_subgraph_shared<1, LOCAL, 1024>, a, 1, threads, bytes, s, grid, limit);
-    else if constexpr (W == 2)
-        return threads <= 256 ? launch_shared(k_subgraph_shared<2, LOCAL, 256>, a, 1, threads, bytes, s, grid, limit)
-                              : launch_shared(k_subgraph_shared<2, LOCAL, 512>, a, 1, threads, bytes, s, grid, limit);
-    else return launch_shared(k_subgraph_shared<W, LOCAL, 256>, a, 1, threads, bytes, s, grid, limit);
+    return launch_shared(k_subgraph_shared<W, LOCAL, local_threads(W)>, a, 1, threads, bytes, s, grid, limit);
 }
 template <int W> int occupancy_local_w(uint32_t threads, size_t bytes) {
-    if constexpr (W == 1) return occupancy_of(k_subgraph_shared<1, LOCAL, 1024>, 1, threads, bytes, max_table_bytes<1>());
-    else if constexpr (W == 2)
-        return threads <= 256 ? occupancy_of(k_subgraph_shared<2, LOCAL, 256>, 1, threads, bytes, max_table_bytes<2>())
-                              : occupancy_of(k_subgraph_shared<2, LOCAL, 512>, 1, threads, bytes, max_table_bytes<2>());
-    else return occupancy_of(k_subgraph_shared<W, LOCAL, 256>, 1, threads, bytes, max_table_bytes<W>());
+    return occupancy_of(k_subgraph_shared<W, LOCAL, local_threads(W)>, 1, threads, bytes, max_table_bytes<W>());
 }
 cudaError_t launch_local(const SubgraphArgs& a, int words, uint32_t threads, size_t bytes, cudaStream_t s, uint32_t grid) {
     switch (words) {

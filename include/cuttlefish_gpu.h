@@ -67,8 +67,8 @@ typedef struct cfg_params {
                                  rebuild of the tables that overflow. */
     uint32_t slots_per_thread; /* one-CTA subgraph tables run slots / slots_per_thread threads (rounded
                                   up to whole warps, at least 64, at most the kernel form's largest
-                                  CTA); 0 = default 4.  8 runs 256-thread CTAs on 2048-slot tables,
-                                  four per SM.  Speed only: results never depend on it. */
+                                  CTA); 0 = chosen with the table's size.  Speed only: results never
+                                  depend on it. */
     uint32_t reserved;
 } cfg_params;
 

@@ -261,3 +261,16 @@ def test_record_merging(case):
     else:
         g = synth.genome_with_repeats(rng, 20_000, n_copies=5, n_pal=3)
         compare(synth.reads(rng, g, 6_000), 31, 20, 2, 256, load_pct=30, extra_flags=cfgpu.CFG_FLAG_NO_RECORD_DEDUP)
+
+
+@pytest.mark.parametrize("k", [31, 63, 95, 127])
+def test_table_shapes(k):
+    """One subgraph filled to either side of the line between every pair of one-CTA table sizes (half load for
+    k <= 31, two thirds beyond) and past the largest."""
+    slots = {31: (64, 128, 256, 520, 1128, 2344, 4096, 8192), 63: (64, 128, 256, 544, 1152, 1760, 2368, 3584, 7200)}.get(
+        k, (64, 128, 256, 560, 1168, 1576, 2384, 4816))
+    rng = np.random.default_rng(60 + k)
+    for s in slots:
+        line = s // 2 if k == 31 else 2 * s // 3          # k-mer instances that still fit
+        for n in (line * 9 // 10, line, line + line // 8 + 1):
+            compare([synth.random_seq(rng, n + k - 1)], k, 20, 1, 1)
