@@ -12,14 +12,18 @@
 // a base, or a break (a non-ACGT character, a record boundary).  The state at
 // each 4 KiB chunk is found by composing the chunks' state-transfer functions
 // (a scan), so every chunk runs independently:
-//   A  transfer function of every chunk (and of every thread's bytes before it, kept
-//      for C, E and G)                              B  scan: each chunk's start state
-//   C  bases and breaks of every chunk (and of every thread's bytes before it in its
-//      chunk, kept for E and G)                     D  scan: each chunk's offsets
+//   A  transfer function of every chunk (and of every group's bytes before it, kept
+//      for C)                                       B  scan: each chunk's start state
+//   C  each group's emissions as two 16-bit masks (kept for E and G), the chunk's bases
+//      and breaks (and those before every group)    D  scan: each chunk's offsets
 //   E  the base rank of every break                F  fragments: lengths, keep, offsets
 //   G  bases written 2 bits each into the packed stream.
-// E and G visit only the threads with breaks, or bases, to place; what one thread does
-// with its 16 bytes is in cfg_parse_thread.cuh.
+// A and C give a warp a whole chunk, 32 groups of 16 bytes at a time: no barrier, every
+// load of the chunk in flight at once, the scan carried in registers.  E and G visit only
+// the groups with breaks, or bases, to place; what is done with a group's 16 bytes is in
+// cfg_parse_thread.cuh.  Bound: instruction issue (the text is read three times, 0.3 ms of
+// the 1.75 ms that 640 MB of FASTQ take; 8.8 ms with a byte-by-byte walk of the groups that
+// hold a newline, CTA-wide scans and one-CTA scans over the chunks).
 #include "cuttlefish_gpu.h"
 #include "cfg_host.h"
 #include "cfg_internal.h"
@@ -38,8 +42,11 @@ struct ParseArgs {
     uint64_t bytes, n_chunks;
     FsmBits fsm;
     uint32_t* chunk_f;             // A: transfer function; B: start state
-    uint16_t* thread_f;            // A: per thread, the chunk's function before the thread's bytes
-    uint32_t* thread_pre;          // C: per thread, the chunk's bases and breaks before the thread's bytes
+    uint16_t* thread_f;            // A: per group, the chunk's function before it
+    uint32_t* thread_pre;          // C: per group, the chunk's bases and breaks before it
+    uint32_t* thread_m;            // C: per group, its bytes that are bases (low half) and breaks (high half)
+    uint32_t* part_f;              // B: transfer function of every 1024 chunks
+    unsigned long long* part_s;    // C: bases and breaks of every 1024 chunks
     unsigned long long* chunk_b;   // C: bases; D: bases before the chunk
     unsigned long long* chunk_k;   // C: breaks; D: breaks before the chunk
     unsigned long long* brk_rank;  // E: bases before break i (NB + 1 entries)
@@ -47,9 +54,12 @@ struct ParseArgs {
     const unsigned long long* frag_out;   // F: output start of fragment i, ~0 if dropped
 };
 
-// The bytes of thread t of a chunk (zero past the end).
-__device__ __forceinline__ Group load_group(const ParseArgs& a, uint64_t chunk) {
-    const uint64_t p = chunk * CHUNK + (uint64_t)threadIdx.x * BPT;
+constexpr uint32_t FULL = 0xffffffffu;
+constexpr uint32_t WARP_GROUPS = TPB / 32;   // groups a lane takes of its warp's chunk: 8
+constexpr uint32_t SCAN_CHUNKS = 1024;       // chunks per CTA of the scans B and D
+
+// The 16 bytes at p (zero past the end).
+__device__ __forceinline__ Group load_group(const ParseArgs& a, uint64_t p) {
     Group g;
     if (p + BPT <= a.bytes) {
         const uint4 w = *(const uint4*)(a.text + p);
@@ -66,154 +76,204 @@ __device__ __forceinline__ Group load_group(const ParseArgs& a, uint64_t chunk) 
     }
     return g;
 }
-
-// Exclusive scan of transfer functions over the CTA (in thread order).
-__device__ uint32_t block_scan_f(uint32_t f, uint32_t n, uint32_t* sh) {
-    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    uint32_t x = f;   // inclusive within the warp
-#pragma unroll
-    for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
-        if (lane >= (uint32_t)d) x = compose(y, x, n);
-    }
-    if (lane == 31) sh[wid] = x;
-    __syncthreads();
-    if (threadIdx.x == 0) {   // 8 warps: compose in order
-        uint32_t run = identity(n);
-        for (uint32_t w = 0; w < TPB / 32; ++w) { const uint32_t t = sh[w]; sh[w] = run; run = compose(run, t, n); }
-        sh[TPB / 32] = run;
-    }
-    __syncthreads();
-    const uint32_t before_warp = sh[wid];
-    uint32_t ex = __shfl_up_sync(0xffffffffu, x, 1);
-    if (lane == 0) ex = identity(n);
-    const uint32_t r = compose(before_warp, ex, n);
-    __syncthreads();
-    return r;
+__device__ __forceinline__ uint32_t bytes_at(const ParseArgs& a, uint64_t p) {   // of the group at p
+    return p >= a.bytes ? 0 : (uint32_t)umin64(BPT, a.bytes - p);
 }
 
-__device__ __forceinline__ uint32_t bytes_of_thread(const ParseArgs& a, uint64_t chunk) {
-    const uint64_t p = chunk * CHUNK + (uint64_t)threadIdx.x * BPT;
-    return p >= a.bytes ? 0 : (uint32_t)umin64(BPT, a.bytes - p);
+__device__ __forceinline__ Fn identity_fn() { return Fn{0x03020100u, 4u}; }
+__device__ __forceinline__ Fn shfl_fn(Fn f, int src) { return Fn{__shfl_sync(FULL, f.lo, src), __shfl_sync(FULL, f.hi, src)}; }
+// Inclusive scan of transfer functions over the warp (in lane order).
+__device__ __forceinline__ Fn warp_scan_fn(Fn x, uint32_t lane) {
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const Fn y{__shfl_up_sync(FULL, x.lo, d), __shfl_up_sync(FULL, x.hi, d)};
+        if (lane >= (uint32_t)d) x = fn_then(y, x);
+    }
+    return x;
 }
 
 // A: the chunk's transfer function.
 __global__ void __launch_bounds__(TPB) k_parse_transfer(ParseArgs a) {
-    __shared__ uint32_t sh[TPB / 32 + 1];
-    for (uint64_t c = blockIdx.x; c < a.n_chunks; c += gridDim.x) {
-        const Group g = load_group(a, c);
-        const uint32_t f = thread_transfer(a.fsm, g, bytes_of_thread(a, c));
-        const uint32_t ex = block_scan_f(f, a.fsm.n, sh);
-        a.thread_f[c * TPB + threadIdx.x] = (uint16_t)ex;
-        if (threadIdx.x == 0) a.chunk_f[c] = sh[TPB / 32];
-        __syncthreads();
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t nw = (uint64_t)gridDim.x * (TPB / 32);
+    for (uint64_t c = (uint64_t)blockIdx.x * (TPB / 32) + (threadIdx.x >> 5); c < a.n_chunks; c += nw) {
+        Group g[WARP_GROUPS];
+#pragma unroll
+        for (uint32_t i = 0; i < WARP_GROUPS; ++i) g[i] = load_group(a, c * CHUNK + (uint64_t)(i * 32 + lane) * BPT);
+        Fn carry = identity_fn();
+#pragma unroll
+        for (uint32_t i = 0; i < WARP_GROUPS; ++i) {
+            const uint32_t t = i * 32 + lane;
+            const Fn x = warp_scan_fn(thread_fn(a.fsm, g[i], bytes_at(a, c * CHUNK + (uint64_t)t * BPT)), lane);
+            const Fn up{__shfl_up_sync(FULL, x.lo, 1), __shfl_up_sync(FULL, x.hi, 1)};
+            a.thread_f[c * TPB + t] = (uint16_t)fn_bits(lane ? fn_then(carry, up) : carry);
+            carry = fn_then(carry, shfl_fn(x, 31));
+        }
+        if (lane == 0) a.chunk_f[c] = fn_bits(carry);
     }
 }
 
-// B (one CTA): chunk transfer functions -> each chunk's start state.
-__global__ void __launch_bounds__(1024) k_parse_states(ParseArgs a) {
-    __shared__ uint32_t fs[1024];
-    const uint32_t n = a.fsm.n;
-    const uint64_t per = (a.n_chunks + 1023) / 1024;
-    const uint64_t c0 = umin64(a.n_chunks, threadIdx.x * per), c1 = umin64(a.n_chunks, c0 + per);
-    uint32_t f = identity(n);
-    for (uint64_t c = c0; c < c1; ++c) f = compose(f, a.chunk_f[c], n);
-    fs[threadIdx.x] = f;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t run = identity(n);
-        for (uint32_t t = 0; t < 1024; ++t) { const uint32_t x = fs[t]; fs[t] = run; run = compose(run, x, n); }
-    }
-    __syncthreads();
-    uint32_t st = f_at(fs[threadIdx.x], a.fsm.start);
-    for (uint64_t c = c0; c < c1; ++c) {
-        const uint32_t tf = a.chunk_f[c];
-        a.chunk_f[c] = st;
-        st = f_at(tf, st);
-    }
-}
-
-// A thread's start state: pass A's prefix from B's start state of the chunk.
-__device__ __forceinline__ uint32_t thread_state(const ParseArgs& a, uint64_t c) {
-    return f_at(a.thread_f[c * TPB + threadIdx.x], a.chunk_f[c]);
-}
-
-__device__ __forceinline__ void block_sum2(uint32_t& x, uint32_t& y, uint32_t* sh, uint32_t& ex_x, uint32_t& ex_y,
-                                           uint32_t& tot_x, uint32_t& tot_y) {
+// The functions of the 4 chunks of this thread (of the CTA's SCAN_CHUNKS) composed, and
+// the exclusive scan of those over the CTA; `all`: the CTA's whole function.
+__device__ __forceinline__ Fn block_scan_fn(Fn f, Fn* sh, Fn& all) {
     const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
-    uint32_t a = x, b = y;
+    const Fn x = warp_scan_fn(f, lane);
+    if (lane == 31) sh[wid] = x;
+    __syncthreads();
+    Fn before = identity_fn();
+    all = identity_fn();
+#pragma unroll
+    for (uint32_t w = 0; w < TPB / 32; ++w) {
+        if (w == wid) before = all;
+        all = fn_then(all, sh[w]);
+    }
+    const Fn up{__shfl_up_sync(FULL, x.lo, 1), __shfl_up_sync(FULL, x.hi, 1)};
+    __syncthreads();
+    return lane ? fn_then(before, up) : before;
+}
+static_assert(SCAN_CHUNKS == 4 * TPB, "a thread takes 4 chunks");
+
+// B, first pass: the transfer function of every SCAN_CHUNKS chunks.
+__global__ void __launch_bounds__(TPB) k_parse_states_sum(ParseArgs a) {
+    __shared__ Fn sh[TPB / 32];
+    const uint64_t c0 = (uint64_t)blockIdx.x * SCAN_CHUNKS + 4 * threadIdx.x;
+    Fn f = identity_fn(), all;
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j)
+        if (c0 + j < a.n_chunks) f = fn_then(f, fn_of(a.chunk_f[c0 + j]));
+    block_scan_fn(f, sh, all);
+    if (threadIdx.x == 0) a.part_f[blockIdx.x] = fn_bits(all);
+}
+
+// B, second pass: each chunk's start state.
+__global__ void __launch_bounds__(TPB) k_parse_states(ParseArgs a) {
+    __shared__ Fn sh[TPB / 32];
+    // the CTAs before this one, a contiguous share per thread
+    const uint32_t per = (blockIdx.x + TPB - 1) / TPB;
+    const uint32_t p0 = min(blockIdx.x, threadIdx.x * per), p1 = min(blockIdx.x, p0 + per);
+    Fn f = identity_fn(), base, all;
+    for (uint32_t p = p0; p < p1; ++p) f = fn_then(f, fn_of(a.part_f[p]));
+    block_scan_fn(f, sh, base);
+    const uint64_t c0 = (uint64_t)blockIdx.x * SCAN_CHUNKS + 4 * threadIdx.x;
+    uint32_t tf[4];
+    f = identity_fn();
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+        tf[j] = c0 + j < a.n_chunks ? a.chunk_f[c0 + j] : 0u;
+        if (c0 + j < a.n_chunks) f = fn_then(f, fn_of(tf[j]));
+    }
+    const Fn ex = block_scan_fn(f, sh, all);
+    uint32_t st = f_at(fn_bits(fn_then(base, ex)), a.fsm.start);
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j)
+        if (c0 + j < a.n_chunks) {
+            a.chunk_f[c0 + j] = st;
+            st = f_at(tf[j], st);
+        }
+}
+
+// C: emissions of every group, bases and breaks of every chunk, and before every group.
+__global__ void __launch_bounds__(TPB) k_parse_counts(ParseArgs a) {
+    const uint32_t lane = threadIdx.x & 31;
+    const uint64_t nw = (uint64_t)gridDim.x * (TPB / 32);
+    for (uint64_t c = (uint64_t)blockIdx.x * (TPB / 32) + (threadIdx.x >> 5); c < a.n_chunks; c += nw) {
+        Group g[WARP_GROUPS];
+        uint32_t tf[WARP_GROUPS];
+#pragma unroll
+        for (uint32_t i = 0; i < WARP_GROUPS; ++i) {
+            g[i] = load_group(a, c * CHUNK + (uint64_t)(i * 32 + lane) * BPT);
+            tf[i] = a.thread_f[c * TPB + i * 32 + lane];
+        }
+        const uint32_t st = a.chunk_f[c];
+        uint32_t carry = 0;   // bases | breaks << 16 before this step's groups (a chunk holds 4096 bytes)
+#pragma unroll
+        for (uint32_t i = 0; i < WARP_GROUPS; ++i) {
+            const uint32_t t = i * 32 + lane;
+            const Emits e = thread_emits(a.fsm, f_at(tf[i], st), g[i], bytes_at(a, c * CHUNK + (uint64_t)t * BPT));
+            const uint32_t own = pre_pack(popc32(e.base), popc32(e.brk));
+            uint32_t x = own;
+#pragma unroll
+            for (int d = 1; d < 32; d <<= 1) {
+                const uint32_t y = __shfl_up_sync(FULL, x, d);
+                if (lane >= (uint32_t)d) x += y;
+            }
+            a.thread_pre[c * TPB + t] = carry + x - own;
+            a.thread_m[c * TPB + t] = e.base | (e.brk << 16);
+            carry += __shfl_sync(FULL, x, 31);
+        }
+        if (lane == 0) {
+            a.chunk_b[c] = pre_bases(carry); a.chunk_k[c] = pre_breaks(carry);
+            unsigned long long* ps = a.part_s + 2 * (c / SCAN_CHUNKS);
+            atomicAdd(ps, (unsigned long long)pre_bases(carry));
+            atomicAdd(ps + 1, (unsigned long long)pre_breaks(carry));
+        }
+    }
+}
+
+// Exclusive scan over the CTA of two sums; their totals in tot.
+__device__ __forceinline__ void block_scan2(unsigned long long& x, unsigned long long& y, unsigned long long (*sh)[2],
+                                            unsigned long long (&tot)[2]) {
+    const uint32_t lane = threadIdx.x & 31, wid = threadIdx.x >> 5;
+    unsigned long long a = x, b = y;
 #pragma unroll
     for (int d = 1; d < 32; d <<= 1) {
-        const uint32_t p = __shfl_up_sync(0xffffffffu, a, d), q = __shfl_up_sync(0xffffffffu, b, d);
+        const unsigned long long p = __shfl_up_sync(FULL, a, d), q = __shfl_up_sync(FULL, b, d);
         if (lane >= (uint32_t)d) { a += p; b += q; }
     }
-    if (lane == 31) { sh[wid] = a; sh[16 + wid] = b; }
+    if (lane == 31) { sh[wid][0] = a; sh[wid][1] = b; }
     __syncthreads();
-    if (threadIdx.x == 0) {
-        uint32_t ra = 0, rb = 0;
-        for (uint32_t w = 0; w < TPB / 32; ++w) {
-            const uint32_t ta = sh[w], tb = sh[16 + w];
-            sh[w] = ra; sh[16 + w] = rb; ra += ta; rb += tb;
+    unsigned long long ba = 0, bb = 0;
+    tot[0] = tot[1] = 0;
+#pragma unroll
+    for (uint32_t w = 0; w < TPB / 32; ++w) {
+        if (w == wid) { ba = tot[0]; bb = tot[1]; }
+        tot[0] += sh[w][0]; tot[1] += sh[w][1];
+    }
+    __syncthreads();
+    x = ba + a - x; y = bb + b - y;
+}
+
+// D: exclusive prefix sums of the chunks' bases and breaks; the last entries (index
+// n_chunks) get the totals.
+__global__ void __launch_bounds__(TPB) k_parse_offsets(ParseArgs a) {
+    __shared__ unsigned long long sh[TPB / 32][2];
+    unsigned long long b = 0, k = 0, base[2], tot[2];
+    for (uint32_t p = threadIdx.x; p < blockIdx.x; p += TPB) { b += a.part_s[2 * p]; k += a.part_s[2 * p + 1]; }
+    block_scan2(b, k, sh, base);
+    const uint64_t c0 = (uint64_t)blockIdx.x * SCAN_CHUNKS + 4 * threadIdx.x;
+    unsigned long long cb[4], ck[4];
+    b = k = 0;
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j) {
+        cb[j] = c0 + j < a.n_chunks ? a.chunk_b[c0 + j] : 0ull;
+        ck[j] = c0 + j < a.n_chunks ? a.chunk_k[c0 + j] : 0ull;
+        b += cb[j]; k += ck[j];
+    }
+    block_scan2(b, k, sh, tot);
+    b += base[0]; k += base[1];
+#pragma unroll
+    for (uint32_t j = 0; j < 4; ++j)
+        if (c0 + j < a.n_chunks) {
+            a.chunk_b[c0 + j] = b; a.chunk_k[c0 + j] = k;
+            b += cb[j]; k += ck[j];
         }
-        sh[8] = ra; sh[24] = rb;
-    }
-    __syncthreads();
-    ex_x = sh[wid] + a - x; ex_y = sh[16 + wid] + b - y;
-    tot_x = sh[8]; tot_y = sh[24];
-    __syncthreads();
-}
-
-// C: bases and breaks of every chunk, and of every thread's bytes before it in its chunk.
-__global__ void __launch_bounds__(TPB) k_parse_counts(ParseArgs a) {
-    __shared__ uint32_t sh[32];
-    for (uint64_t c = blockIdx.x; c < a.n_chunks; c += gridDim.x) {
-        const Group g = load_group(a, c);
-        uint32_t nb, nk, eb, ek, tb, tk;
-        thread_counts(a.fsm, thread_state(a, c), g, bytes_of_thread(a, c), nb, nk);
-        block_sum2(nb, nk, sh, eb, ek, tb, tk);
-        a.thread_pre[c * TPB + threadIdx.x] = pre_pack(eb, ek);
-        if (threadIdx.x == 0) { a.chunk_b[c] = tb; a.chunk_k[c] = tk; }
+    if (blockIdx.x == gridDim.x - 1 && threadIdx.x == 0) {
+        a.chunk_b[a.n_chunks] = base[0] + tot[0];
+        a.chunk_k[a.n_chunks] = base[1] + tot[1];
     }
 }
 
-// D (one CTA): exclusive prefix sums of the chunks' bases and breaks; the last
-// entries (index n_chunks) get the totals.
-__global__ void __launch_bounds__(1024) k_parse_offsets(ParseArgs a) {
-    __shared__ unsigned long long sb[1024], sk[1024];
-    const uint64_t per = (a.n_chunks + 1023) / 1024;
-    const uint64_t c0 = umin64(a.n_chunks, threadIdx.x * per), c1 = umin64(a.n_chunks, c0 + per);
-    unsigned long long b = 0, k = 0;
-    for (uint64_t c = c0; c < c1; ++c) { b += a.chunk_b[c]; k += a.chunk_k[c]; }
-    sb[threadIdx.x] = b; sk[threadIdx.x] = k;
-    __syncthreads();
-    if (threadIdx.x == 0) {
-        unsigned long long rb = 0, rk = 0;
-        for (uint32_t t = 0; t < 1024; ++t) {
-            const unsigned long long x = sb[t], y = sk[t];
-            sb[t] = rb; sk[t] = rk; rb += x; rk += y;
-        }
-        a.chunk_b[a.n_chunks] = rb; a.chunk_k[a.n_chunks] = rk;
-    }
-    __syncthreads();
-    unsigned long long rb = sb[threadIdx.x], rk = sk[threadIdx.x];
-    for (uint64_t c = c0; c < c1; ++c) {
-        const unsigned long long x = a.chunk_b[c], y = a.chunk_k[c];
-        a.chunk_b[c] = rb; a.chunk_k[c] = rk;
-        rb += x; rk += y;
-    }
-}
-
-__device__ __forceinline__ ThreadSpan thread_span(const ParseArgs& a, uint64_t c) {
-    return parse::thread_span(a.thread_pre, a.chunk_b, a.chunk_k, c, threadIdx.x);
-}
+__device__ __forceinline__ Emits group_emits(uint32_t m) { return Emits{m & 0xFFFFu, m >> 16}; }
 
 // E: for every break, the number of bases before it; break NB (after the text) closes
-// the last fragment.  Only threads whose bytes emit a break read them.
+// the last fragment.  Only groups that emit a break are looked at.
 __global__ void __launch_bounds__(TPB) k_parse_breaks(ParseArgs a) {
-    for (uint64_t c = blockIdx.x; c < a.n_chunks; c += gridDim.x) {
-        const ThreadSpan sp = thread_span(a, c);
-        if (sp.nk == 0) continue;
-        thread_breaks(a.fsm, thread_state(a, c), load_group(a, c), bytes_of_thread(a, c), sp.r, sp.kk, a.brk_rank);
+    const uint64_t n = a.n_chunks * TPB, stride = (uint64_t)gridDim.x * TPB;
+    for (uint64_t i = (uint64_t)blockIdx.x * TPB + threadIdx.x; i < n; i += stride) {
+        const Emits e = group_emits(a.thread_m[i]);
+        if (!e.brk) continue;
+        const uint32_t pre = a.thread_pre[i];
+        emit_breaks(e, a.chunk_b[i / TPB] + pre_bases(pre), a.chunk_k[i / TPB] + pre_breaks(pre), a.brk_rank);
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) a.brk_rank[a.chunk_k[a.n_chunks]] = a.chunk_b[a.n_chunks];
 }
@@ -328,13 +388,15 @@ struct AtomicOr64 {
 };
 
 // G: every kept base to its place in the packed stream (MSB-first, 32 per word).  Only
-// threads whose bytes emit a base read them.
+// groups that emit a base read their bytes.
 __global__ void __launch_bounds__(TPB) k_parse_pack(ParseArgs a) {
-    for (uint64_t c = blockIdx.x; c < a.n_chunks; c += gridDim.x) {
-        const ThreadSpan sp = thread_span(a, c);
-        if (sp.nb == 0) continue;
-        thread_pack(a.fsm, thread_state(a, c), load_group(a, c), bytes_of_thread(a, c), sp.r, sp.kk, sp.nb, sp.nk,
-                    a.frag_out, a.brk_rank, a.packed, AtomicOr64{});
+    const uint64_t n = a.n_chunks * TPB, stride = (uint64_t)gridDim.x * TPB;
+    for (uint64_t i = (uint64_t)blockIdx.x * TPB + threadIdx.x; i < n; i += stride) {
+        const Emits e = group_emits(a.thread_m[i]);
+        if (!e.base) continue;
+        const uint32_t pre = a.thread_pre[i];
+        emit_pack(e, load_group(a, i * BPT), a.chunk_b[i / TPB] + pre_bases(pre), a.chunk_k[i / TPB] + pre_breaks(pre),
+                  a.frag_out, a.brk_rank, a.packed, AtomicOr64{});
     }
 }
 
@@ -348,14 +410,18 @@ int parse_text_device(const uint8_t* d_text, uint64_t bytes, int fastq, uint32_t
     const uint64_t nc = a.n_chunks;
     if (!pb.ensure_chunks(nc + 1)) return CFG_ERR_OOM;
     a.chunk_f = pb.chunk_f; a.chunk_b = pb.chunk_b; a.chunk_k = pb.chunk_k; a.thread_f = pb.thread_f;
-    a.thread_pre = pb.thread_pre;
-    const unsigned grid = (unsigned)std::min<uint64_t>(std::max<uint64_t>(nc, 1), 148ull * 16);
+    a.thread_pre = pb.thread_pre; a.thread_m = pb.thread_m; a.part_f = pb.chunk_part_f; a.part_s = pb.chunk_part_s;
+    const unsigned wgrid = (unsigned)std::min<uint64_t>((nc + TPB / 32 - 1) / (TPB / 32), 148ull * 32);   // a warp per chunk
+    const unsigned grid = (unsigned)std::min<uint64_t>(std::max<uint64_t>(nc, 1), 148ull * 32);           // a thread per group
+    const unsigned sgrid = (unsigned)std::max<uint64_t>((nc + SCAN_CHUNKS - 1) / SCAN_CHUNKS, 1);
+    if (cudaMemsetAsync(a.part_s, 0, 16ull * sgrid, s) != cudaSuccess) return CFG_ERR_CUDA;
     if (nc) {
-        k_parse_transfer<<<grid, TPB, 0, s>>>(a);
-        k_parse_states<<<1, 1024, 0, s>>>(a);
-        k_parse_counts<<<grid, TPB, 0, s>>>(a);
+        k_parse_transfer<<<wgrid, TPB, 0, s>>>(a);
+        k_parse_states_sum<<<sgrid, TPB, 0, s>>>(a);
+        k_parse_states<<<sgrid, TPB, 0, s>>>(a);
+        k_parse_counts<<<wgrid, TPB, 0, s>>>(a);
     }
-    k_parse_offsets<<<1, 1024, 0, s>>>(a);
+    k_parse_offsets<<<sgrid, TPB, 0, s>>>(a);
     unsigned long long tot[2] = {0, 0};   // bases, breaks
     if (cudaMemcpyAsync(&tot[0], a.chunk_b + nc, 8, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
         cudaMemcpyAsync(&tot[1], a.chunk_k + nc, 8, cudaMemcpyDeviceToHost, s) != cudaSuccess ||

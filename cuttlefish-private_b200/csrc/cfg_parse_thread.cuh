@@ -7,10 +7,12 @@
 // machine over the classes (the line structure of FASTA or FASTQ) gives each byte an
 // emission: skipped, a base, or a break (a non-ACGT character, a record boundary).
 //
-// Most 16-byte groups of a real file lie inside one line -- bases of a sequence line,
-// quality letters, a header -- where the state loops on every byte.  For those the
-// counts, the transfer function and the 2-bit codes come from word-wise byte compares
-// (SWAR) instead of a walk of the FSM byte by byte; every other group takes the walk.
+// A group is never walked byte by byte.  In both machines a run of base and other bytes
+// moves every state once (one class map, idempotent) and emits alike from its first byte to
+// its last -- bases and breaks from the states of a sequence line, nothing from the others
+// -- so only the delimiters ('\n', '\r', and '>' where it is one) step the state.  Word-wise
+// byte compares (SWAR) find them and the base letters as 16-bit masks; the group's emissions
+// are two such masks, and its 2-bit codes are cut out of all 16 bytes' codes by runs.
 #pragma once
 
 #include <cstdint>
@@ -28,6 +30,31 @@ constexpr uint32_t CHUNK = 4096, TPB = 256, BPT = CHUNK / TPB;   // bytes per th
 enum : uint32_t { C_NL = 0, C_GT = 1, C_BASE = 2, C_CR = 3, C_OTHER = 4, NCLASS = 5 };
 enum : uint32_t { E_SKIP = 0, E_BASE = 1, E_BREAK = 2 };
 
+CFG_PHD uint32_t byte_perm(uint32_t x, uint32_t y, uint32_t s) {   // bytes of {y, x} picked by s's four nibbles
+#ifdef __CUDA_ARCH__
+    return __byte_perm(x, y, s);
+#else
+    const uint64_t v = ((uint64_t)y << 32) | x;
+    uint32_t r = 0;
+    for (int i = 0; i < 4; ++i) r |= (uint32_t)(v >> (8 * ((s >> (4 * i)) & 7)) & 0xFF) << (8 * i);
+    return r;
+#endif
+}
+// A transfer function of at most 5 states as bytes: state s's image in byte s of lo, state
+// 4's in the low byte of hi (the rest of hi is unspecified).
+struct Fn { uint32_t lo, hi; };
+CFG_PHD Fn fn_of(uint32_t f) {   // from 3 bits per state
+    return Fn{(f & 7u) | ((f << 5) & 0x700u) | ((f << 10) & 0x70000u) | ((f << 15) & 0x7000000u), (f >> 12) & 7u};
+}
+CFG_PHD uint32_t fn_bits(Fn f) {   // to 3 bits per state
+    return (f.lo & 7u) | ((f.lo >> 5) & 0x38u) | ((f.lo >> 10) & 0x1C0u) | ((f.lo >> 15) & 0xE00u) | ((f.hi & 7u) << 12);
+}
+// first f, then g: f's images, as nibbles, are the byte selectors into g
+CFG_PHD Fn fn_then(Fn f, Fn g) {
+    const uint32_t y = f.lo | (f.lo >> 4);
+    return Fn{byte_perm(g.lo, g.hi, byte_perm(y, 0, 0x4420u)), byte_perm(g.lo, g.hi, f.hi & 7u)};
+}
+
 // The tables of an FSM of at most 5 states packed into registers: entry (class c, state s)
 // at index i = 5 c + s, its next state in 3 bits (bits 3i.. of nx_lo for i < 21, of nx_hi
 // above) and its emission in 2 bits of em.  A lookup is a few shifts on values every
@@ -36,16 +63,17 @@ enum : uint32_t { E_SKIP = 0, E_BASE = 1, E_BREAK = 2 };
 struct FsmBits {
     unsigned long long nx_lo, nx_hi, em;
     // class c's whole next-state map as a transfer function (3 bits per state): bits 15c..
-    // of cf_lo for c < 4, cf_hi for c = 4; idem bit c: that map is idempotent (a run of
-    // class-c bytes acts as one)
+    // of cf_lo for c < 4, cf_hi for c = 4
     unsigned long long cf_lo;
-    uint32_t cf_hi, idem;
+    uint32_t cf_hi;
     uint32_t n, start;
     // word-wise groups: loop_mask bit s -- state s stays s on a base and on an other byte;
     // gt_other -- '>' has the next states and emissions of an other byte in every state
     // (it is then no delimiter); bo_idem -- bases and other bytes have one class map, and
-    // it is idempotent (a group of them composes to that map)
-    uint32_t loop_mask, gt_other, bo_idem;
+    // it is idempotent (a group of them composes to that map); seq_mask bit s -- runs that
+    // start in state s emit (base: E_BASE, other: E_BREAK; from the other states E_SKIP)
+    uint32_t loop_mask, gt_other, bo_idem, seq_mask;
+    Fn run, nl, cr, gt;   // the class maps of a run, '\n', '\r' and '>'
 };
 
 CFG_PHD uint32_t fsm_next(const FsmBits& f, uint32_t st, uint32_t cl) {
@@ -103,91 +131,126 @@ CFG_PHD uint32_t eq_bytes(uint32_t x, uint32_t b) {
     return ~(((y & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | y) & 0x80808080u;
 }
 
-// Whether the group holds a newline, a '\r' or -- unless it acts as an other byte -- a '>'.
-CFG_PHD bool has_delimiter(const FsmBits& f, const Group& g) {
+// The top bits of x's four bytes as bits 0..3.
+CFG_PHD uint32_t top_bits(uint32_t x) { return ((x & 0x80808080u) * 0x00204081u) >> 28; }
+
+// Whether the group may hold a delimiter: some byte below 0x0E ('\n' and '\r' are) or,
+// unless it acts as an other byte, a '>'.
+CFG_PHD bool maybe_delimiter(const FsmBits& f, const Group& g) {
     uint32_t m = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        m |= eq_bytes(g.w[i], '\n') | eq_bytes(g.w[i], '\r');
-        if (!f.gt_other) m |= eq_bytes(g.w[i], '>');
+        m |= (g.w[i] - 0x0E0E0E0Eu) & ~g.w[i];
+        if (!f.gt_other) {
+            const uint32_t y = g.w[i] ^ 0x3E3E3E3Eu;
+            m |= (y - 0x01010101u) & ~y;
+        }
     }
-    return m != 0;
+    return (m & 0x80808080u) != 0;
 }
-
-// Base letters (ACGT, either case) among the group's bytes.
-CFG_PHD uint32_t count_acgt(const Group& g) {
-    uint32_t n = 0;
+// Bit i: byte i equals b.
+CFG_PHD uint32_t eq_mask(const Group& g, uint32_t b) {
+    uint32_t m = 0;
+#pragma unroll
+    for (int i = 0; i < 4; ++i) m |= top_bits(eq_bytes(g.w[i], b)) << (4 * i);
+    return m;
+}
+// The delimiters among the group's first nb bytes, by kind.
+struct Delims { uint32_t nl, cr, gt; };
+CFG_PHD Delims delims(const FsmBits& f, const Group& g, uint32_t nb) {
+    const uint32_t v = nb >= BPT ? 0xFFFFu : (1u << nb) - 1u;
+    return Delims{eq_mask(g, '\n') & v, eq_mask(g, '\r') & v, f.gt_other ? 0u : eq_mask(g, '>') & v};
+}
+// Each byte's 2-bit code ((c >> 1) ^ (c >> 2)) & 3: a base letter's (A 0x41, C 0x43, G 0x47,
+// T 0x54 and their lower-case forms: A0 C1 G2 T3), any value for other bytes.
+CFG_PHD uint32_t codes4(uint32_t w) { return ((w >> 1) ^ (w >> 2)) & 0x03030303u; }
+// Bit i: byte i is a base letter -- the letter of its code, either case.
+CFG_PHD uint32_t acgt_mask(const Group& g) {
+    uint32_t m = 0;
 #pragma unroll
     for (int i = 0; i < 4; ++i) {
-        const uint32_t u = g.w[i] & 0xDFDFDFDFu;
-        n += popc32(eq_bytes(u, 'A') | eq_bytes(u, 'C') | eq_bytes(u, 'G') | eq_bytes(u, 'T'));
+        const uint32_t c = codes4(g.w[i]), y = c | (c >> 4);
+        const uint32_t letter = byte_perm(0x54474341u, 0, byte_perm(y, 0, 0x4420u));
+        const uint32_t d = (g.w[i] ^ letter) & 0xDFDFDFDFu;
+        m |= top_bits(~(((d & 0x7F7F7F7Fu) + 0x7F7F7F7Fu) | d)) << (4 * i);
     }
-    return n;
+    return m;
 }
 
-// The transfer function of nb bytes (nb <= 16): the class maps composed in byte order, a
-// run of one idempotent class composed once; a full group without delimiters is one
-// composition when bases and other bytes share an idempotent map.
-CFG_PHD uint32_t thread_transfer(const FsmBits& f, const Group& g, uint32_t nb) {
-    if (nb == BPT && f.bo_idem && !has_delimiter(f, g)) return class_fn(f, C_BASE);
-    uint32_t fn = identity(f.n), prev = NCLASS;
-#pragma unroll
-    for (uint32_t i = 0; i < BPT; ++i) {
-        if (i >= nb) break;
-        const uint32_t cl = byte_class(byte_at(g, i));
-        if (cl != prev || !((f.idem >> cl) & 1)) fn = compose(fn, class_fn(f, cl), f.n);
-        prev = cl;
+CFG_PHD uint32_t low_bit(uint32_t x) {   // index of the lowest set bit (x != 0)
+#ifdef __CUDA_ARCH__
+    return (uint32_t)__ffs((int)x) - 1u;
+#else
+    return (uint32_t)__builtin_ctz(x);
+#endif
+}
+
+// The transfer function of nb bytes (nb <= 16): the runs' map and the delimiters', in order.
+CFG_PHD Fn thread_fn(const FsmBits& f, const Group& g, uint32_t nb) {
+    if (nb == BPT && !maybe_delimiter(f, g)) return f.run;
+    const Delims d = delims(f, g, nb);
+    Fn fn = Fn{0x03020100u, 4u};
+    uint32_t pos = 0;
+    for (uint32_t m = d.nl | d.cr | d.gt; m; m &= m - 1) {
+        const uint32_t p = low_bit(m), b = m & (0u - m);
+        if (p > pos) fn = fn_then(fn, f.run);
+        fn = fn_then(fn, d.nl & b ? f.nl : d.cr & b ? f.cr : f.gt);
+        pos = p + 1;
     }
+    if (nb > pos) fn = fn_then(fn, f.run);
     return fn;
+}
+CFG_PHD uint32_t thread_transfer(const FsmBits& f, const Group& g, uint32_t nb) { return fn_bits(thread_fn(f, g, nb)); }
+
+// What the group's nbytes bytes emit from state st: bit i of base (brk) -- byte i is a base
+// (a break).
+struct Emits { uint32_t base, brk; };
+CFG_PHD Emits thread_emits(const FsmBits& f, uint32_t st, const Group& g, uint32_t nbytes) {
+    if (nbytes == BPT && !maybe_delimiter(f, g)) {
+        if (!((f.seq_mask >> st) & 1)) return Emits{0u, 0u};
+        const uint32_t a = acgt_mask(g);
+        return Emits{a, a ^ 0xFFFFu};
+    }
+    const Delims d = delims(f, g, nbytes);
+    uint32_t seq = 0, brk = 0, pos = 0;   // bytes of emitting runs; breaking delimiters
+    for (uint32_t m = d.nl | d.cr | d.gt; m; m &= m - 1) {
+        const uint32_t p = low_bit(m), b = m & (0u - m);
+        if (p > pos) {
+            if ((f.seq_mask >> st) & 1) seq |= b - (1u << pos);
+            st = f_at(class_fn(f, C_BASE), st);
+        }
+        const uint32_t cl = d.nl & b ? (uint32_t)C_NL : d.cr & b ? (uint32_t)C_CR : (uint32_t)C_GT;
+        if (fsm_emit(f, st, cl) == E_BREAK) brk |= b;
+        st = fsm_next(f, st, cl);
+        pos = p + 1;
+    }
+    if (nbytes > pos && ((f.seq_mask >> st) & 1)) seq |= (1u << nbytes) - (1u << pos);
+    if (!seq) return Emits{0u, brk};
+    const uint32_t a = acgt_mask(g);
+    return Emits{a & seq, brk | (seq & ~a)};
 }
 
 // Bases and breaks the group emits from state st.
 CFG_PHD void thread_counts(const FsmBits& f, uint32_t st, const Group& g, uint32_t nbytes, uint32_t& nb, uint32_t& nk) {
-    if (nbytes == BPT && ((f.loop_mask >> st) & 1) && !has_delimiter(f, g)) {
-        // the state stays st on every byte: bases and other bytes emit one kind each
-        const uint32_t eb = fsm_emit(f, st, C_BASE), eo = fsm_emit(f, st, C_OTHER);
-        const uint32_t na = eb == eo ? BPT : count_acgt(g), no = BPT - na;
-        nb = (eb == E_BASE ? na : 0u) + (eo == E_BASE ? no : 0u);
-        nk = (eb == E_BREAK ? na : 0u) + (eo == E_BREAK ? no : 0u);
-        return;
-    }
-    nb = nk = 0;
-#pragma unroll
-    for (uint32_t i = 0; i < BPT; ++i) {
-        if (i >= nbytes) break;
-        const uint32_t cl = byte_class(byte_at(g, i));
-        const uint32_t e = fsm_emit(f, st, cl);
-        nb += e == E_BASE; nk += e == E_BREAK;
-        st = fsm_next(f, st, cl);
-    }
+    const Emits e = thread_emits(f, st, g, nbytes);
+    nb = popc32(e.base); nk = popc32(e.brk);
 }
 
 // The rank (bases before it) of each break the group emits: r bases and kk breaks precede
 // the group's first byte.
+CFG_PHD void emit_breaks(Emits e, unsigned long long r, unsigned long long kk, unsigned long long* brk_rank) {
+    for (uint32_t m = e.brk; m; m &= m - 1) brk_rank[kk++] = r + popc32(e.base & ((m & (0u - m)) - 1u));
+}
 CFG_PHD void thread_breaks(const FsmBits& f, uint32_t st, const Group& g, uint32_t nbytes, unsigned long long r,
                            unsigned long long kk, unsigned long long* brk_rank) {
-#pragma unroll
-    for (uint32_t i = 0; i < BPT; ++i) {
-        if (i >= nbytes) break;
-        const uint32_t cl = byte_class(byte_at(g, i));
-        const uint32_t e = fsm_emit(f, st, cl);
-        if (e == E_BASE) ++r;
-        else if (e == E_BREAK) brk_rank[kk++] = r;
-        st = fsm_next(f, st, cl);
-    }
+    emit_breaks(thread_emits(f, st, g, nbytes), r, kk, brk_rank);
 }
 
-// 2-bit codes (A0 C1 G2 T3) of 16 base letters of either case, byte 0's in bits 31:30:
-// ((c >> 1) ^ (c >> 2)) & 3 is a letter's code (A 0x41, C 0x43, G 0x47, T 0x54 and
-// their lower-case forms), and the masks keep each byte's code inside its byte.
+// 2-bit codes of the group's 16 bytes, byte 0's in bits 31:30.
 CFG_PHD uint32_t pack16(const Group& g) {
     uint32_t p = 0;
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
-        const uint32_t c = ((g.w[i] >> 1) ^ (g.w[i] >> 2)) & 0x03030303u;
-        const uint32_t q = ((c & 3u) << 6) | (((c >> 8) & 3u) << 4) | (((c >> 16) & 3u) << 2) | ((c >> 24) & 3u);
-        p = (p << 8) | q;
-    }
+    for (int i = 0; i < 4; ++i) p = (p << 8) | ((codes4(g.w[i]) * 0x40100401u) >> 24);
     return p;
 }
 
@@ -201,47 +264,48 @@ CFG_PHD FragPos frag_pos(const unsigned long long* frag_out, const unsigned long
 }
 
 // The group's bases into the packed stream (MSB-first, 32 per word, every word zero
-// before the pass): r bases and kk breaks precede the group; nb and nk are the group's
-// own counts.  or64(word pointer, bits) merges bits into a word (an atomic on the GPU:
-// a word's bases may come from two threads).
+// before the pass): r bases and kk breaks precede the group.  or64(word pointer, bits)
+// merges bits into a word (an atomic on the GPU: a word's bases may come from two threads).
+// Each stretch of bases between two breaks is one fragment's: its runs of adjacent bytes
+// are cut out of the 16 codes, joined, and merged into at most two words.
+template <class Or64>
+CFG_PHD void emit_pack(Emits e, const Group& g, unsigned long long r, unsigned long long kk,
+                       const unsigned long long* frag_out, const unsigned long long* brk_rank, uint64_t* packed, Or64 or64) {
+    const uint64_t codes = (uint64_t)pack16(g) << 32;   // byte 0's at bits 63:62
+    uint32_t brk = e.brk;
+    for (uint32_t left = e.base; left;) {
+        const uint32_t b = brk & (0u - brk);                         // the next break, 0: none
+        uint32_t part = b ? left & (b - 1u) : left;                  // bases before it
+        left ^= part;
+        brk ^= b;
+        if (part) {
+            const FragPos fp = frag_pos(frag_out, brk_rank, kk);
+            const uint32_t total = popc32(part);
+            if (fp.out != ~0ull) {
+                uint64_t acc = 0;
+                uint32_t n = 0;
+                while (part) {
+                    const uint32_t lo = low_bit(part), len = low_bit(~(part >> lo));
+                    acc |= ((codes << (2 * lo)) & ~(~0ull >> (2 * len))) >> (2 * n);   // len <= 16
+                    n += len;
+                    part &= ~(((1u << len) - 1u) << lo);
+                }
+                const unsigned long long q = fp.out + (r - fp.first);
+                const uint32_t o = (uint32_t)(q & 31);
+                or64(packed + (q >> 5), acc >> (2 * o));
+                if (o + n > 32) or64(packed + (q >> 5) + 1, acc << (64 - 2 * o));
+            }
+            r += total;
+        }
+        ++kk;
+    }
+}
 template <class Or64>
 CFG_PHD void thread_pack(const FsmBits& f, uint32_t st, const Group& g, uint32_t nbytes, unsigned long long r,
                          unsigned long long kk, uint32_t nb, uint32_t nk, const unsigned long long* frag_out,
                          const unsigned long long* brk_rank, uint64_t* packed, Or64 or64) {
-    if (nb == 0) return;
-    FragPos fp = frag_pos(frag_out, brk_rank, kk);
-    if (nb == BPT && nk == 0) {   // 16 bases of one fragment, in a row
-        if (fp.out == ~0ull) return;
-        const unsigned long long q = fp.out + (r - fp.first);
-        const uint64_t s = (uint64_t)pack16(g) << 32;   // byte 0's base at bits 63:62
-        const uint32_t o = (uint32_t)(q & 31);
-        or64(packed + (q >> 5), s >> (2 * o));
-        if (o > 16) or64(packed + (q >> 5) + 1, s << (64 - 2 * o));
-        return;
-    }
-    uint64_t word = ~0ull, acc = 0;
-#pragma unroll
-    for (uint32_t i = 0; i < BPT; ++i) {
-        if (i >= nbytes) break;
-        const uint32_t ch = byte_at(g, i), cl = byte_class(ch);
-        const uint32_t e = fsm_emit(f, st, cl);
-        if (e == E_BASE) {
-            if (fp.out != ~0ull) {
-                const unsigned long long q = fp.out + (r - fp.first);
-                const uint64_t w = q >> 5;
-                if (w != word) {
-                    if (word != ~0ull) or64(packed + word, acc);
-                    word = w; acc = 0;
-                }
-                acc |= (uint64_t)base_code(ch) << (62 - 2 * (q & 31));
-            }
-            ++r;
-        } else if (e == E_BREAK) {
-            fp = frag_pos(frag_out, brk_rank, ++kk);
-        }
-        st = fsm_next(f, st, cl);
-    }
-    if (word != ~0ull) or64(packed + word, acc);
+    (void)nk;
+    if (nb) emit_pack(thread_emits(f, st, g, nbytes), g, r, kk, frag_out, brk_rank, packed, or64);
 }
 
 // A thread's exclusive prefix of bases (low 16 bits) and breaks (high 16 bits) within its
@@ -285,17 +349,14 @@ inline FsmBits pack_fsm(const Fsm& m) {
     b.n = m.n; b.start = m.start;
     for (uint32_t c = 0; c < NCLASS; ++c) {
         uint32_t F = 0;
-        bool idem = true;
         for (uint32_t st = 0; st < m.n; ++st) {
             const uint32_t i = 5 * c + st;
             if (i < 21) b.nx_lo |= (unsigned long long)m.next[st][c] << (3 * i);
             else b.nx_hi |= (unsigned long long)m.next[st][c] << (3 * (i - 21));
             b.em |= (unsigned long long)m.emit[st][c] << (2 * i);
             F |= (uint32_t)m.next[st][c] << (3 * st);
-            idem = idem && m.next[m.next[st][c]][c] == m.next[st][c];
         }
         if (c < 4) b.cf_lo |= (unsigned long long)F << (15 * c); else b.cf_hi = F;
-        if (idem) b.idem |= 1u << c;
     }
     // word-wise groups (cfg_parse_thread.cuh): states that loop on bases and other bytes,
     // '>' as an other byte, and one idempotent map for bases and other bytes
@@ -306,7 +367,10 @@ inline FsmBits pack_fsm(const Fsm& m) {
         if (m.next[st][C_GT] != m.next[st][C_OTHER] || m.emit[st][C_GT] != m.emit[st][C_OTHER]) b.gt_other = 0;
         if (m.next[st][C_BASE] != m.next[st][C_OTHER] || m.next[m.next[st][C_BASE]][C_BASE] != m.next[st][C_BASE])
             b.bo_idem = 0;
+        if (m.emit[st][C_BASE] == E_BASE) b.seq_mask |= 1u << st;
     }
+    b.run = fn_of(class_fn(b, C_BASE)); b.nl = fn_of(class_fn(b, C_NL));
+    b.cr = fn_of(class_fn(b, C_CR)); b.gt = fn_of(class_fn(b, C_GT));
     return b;
 }
 

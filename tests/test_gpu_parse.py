@@ -146,3 +146,15 @@ def test_text_timings():
         cx.submit_text(text)
         copy_ms, parse_ms = cx.text_timings()
         assert 0.0 <= copy_ms < 60_000 and 0.0 < parse_ms < 60_000
+
+
+@pytest.mark.parametrize("fastq", [False, True])
+@pytest.mark.parametrize("size", [1, 16, 4095, 4097, (1 << 22) - 1, 1 << 22, (1 << 22) + 1, 3 * (1 << 22) + 4113])
+def test_chunk_edges(fastq, size):
+    """Texts cut at the edges of a 16-byte group, a 4 KiB chunk and the 1024 chunks of a scan block (4 MiB)."""
+    rng = np.random.default_rng(size + fastq)
+    if fastq:
+        piece = fastq_text(rng, 31, 1500)
+    else:
+        piece = b">a\n" + b"".join(synth.random_seq(rng, 70).encode() + b"\n" for _ in range(4000)) + b"NN\r\n>b c\n\nacgt\n"
+    check((piece * (size // len(piece) + 1))[:size], 31)
