@@ -128,6 +128,7 @@ struct UnitigInput {
 // ... the buffers it works in ...
 struct UnitigBuffers {
     DevBuf b_label, b_tab, b_partner, b_X0, b_X1, b_fin, b_off, b_words, b_out, b_job, b_flip, b_sx, b_sw, b_len, b_ends;
+    HostBuf h_words;              // page-locked copy of the collation's result words
     ulonglong2* ends = nullptr;   // both ends of each gathered lm-tig, packed for the pairing pass
     uint32_t end_words = 2;       // 64-bit words per end there: 2 for k <= 63, 4 beyond (set from k)
     uint32_t* len = nullptr;   // each gathered lm-tig's label length (the kernels after the gather read 4 bytes, not a record)
@@ -154,11 +155,12 @@ struct UnitigBuffers {
         DevBuf* all[] = {&b_label, &b_tab, &b_partner, &b_X0, &b_X1, &b_fin, &b_off, &b_words, &b_out, &b_job,
                          &b_flip, &b_sx, &b_sw, &b_len, &b_ends};
         for (DevBuf* b : all) b->release();
+        h_words.release();
     }
 };
 // ... and what it produced: `bytes` of FASTA records at out, the unitigs among them,
 // and how many lm-tigs are left on closed chains (collate_cycles_on_device joins them).
-struct UnitigResult { uint64_t bytes, n_units, n_cycle_lmtigs; uint32_t rounds; };
+struct UnitigResult { uint64_t bytes, n_units, n_cycle_lmtigs; };
 int collate_device(const UnitigInput& in, UnitigBuffers& ub, cudaStream_t s, UnitigResult& res);
 // The m lm-tigs on closed chains (fin == NONE after collate_device) joined into cycles on
 // the device, each written rotated to its canonical start: out_bytes of FASTA records at

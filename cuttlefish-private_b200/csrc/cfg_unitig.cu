@@ -306,30 +306,47 @@ __global__ void __launch_bounds__(256) k_rs_walk(const uint32_t* __restrict__ sx
     atomicOr(err, DERR_WALK_LIMIT);   // step bound exceeded
 }
 
-// One pointer-jumping round over the splitters (double-buffered); counts the entries
-// still unresolved.
-__global__ void k_ut_rank_round(const unsigned long long* __restrict__ n_split, const RankRec* __restrict__ X,
-                                RankRec* X2, unsigned long long* active) {
+// An invalid graph stops the passes after it: no record is reserved or written.
+__device__ __forceinline__ bool failed(const uint32_t* err) { return *err & (DERR_BAD_GRAPH | DERR_WALK_LIMIT); }
+
+// Pointer-jumping rounds over the splitters are queued without a look at how many it takes:
+// act[r] counts the entries still unresolved after round r, and a round does nothing once
+// none is, or once a round resolved none (what is left lies on closed chains; an open chain
+// resolves some entries in every round).
+constexpr uint32_t MAX_ROUNDS = 34;
+__device__ __forceinline__ bool round_runs(const unsigned long long* act, uint32_t r) {
+    return r == 0 || (act[r - 1] && !(r > 1 && act[r - 1] == act[r - 2]));
+}
+// One round (double-buffered by its parity); counts the entries still unresolved.
+__global__ void k_ut_rank_round(const unsigned long long* __restrict__ n_split, RankRec* Xa, RankRec* Xb,
+                                unsigned long long* act, uint32_t round, const uint32_t* __restrict__ err) {
+    if (failed(err) || !round_runs(act, round)) return;
+    const RankRec* X = round & 1 ? Xb : Xa;
+    RankRec* X2 = round & 1 ? Xa : Xb;
     const uint64_t n2 = *n_split;
-    uint32_t act = 0;
+    uint32_t active = 0;
     for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n2; x += (uint64_t)gridDim.x * blockDim.x) {
         RankRec r = X[x];
         if (r.P != NONE) {   // one 16-byte gather of the predecessor's record
             const RankRec q = X[r.P];
             r.P = q.P; r.R = q.R; r.A += q.A;
-            act += q.P != NONE;
+            active += q.P != NONE;
         }
         X2[x] = r;
     }
-    if (!active) return;
-    for (int d = 16; d; d >>= 1) act += __shfl_down_sync(0xffffffffu, act, d);
-    if ((threadIdx.x & 31) == 0 && act) atomicAdd(active, (unsigned long long)act);
+    for (int d = 16; d; d >>= 1) active += __shfl_down_sync(0xffffffffu, active, d);
+    if ((threadIdx.x & 31) == 0 && active) atomicAdd(act + round, (unsigned long long)active);
 }
 
 // 2c: every entry's rank from its splitter's: head entry and bases before it.  Entries
 // on closed chains keep a predecessor (P != NONE); entries no walk passed are on closed
 // chains without a splitter.
-__global__ void k_rs_final(uint64_t n2, const uint2* __restrict__ node, RankRec* X, const RankRec* __restrict__ S) {
+__global__ void k_rs_final(uint64_t n2, const uint2* __restrict__ node, RankRec* X, const RankRec* Sa, const RankRec* Sb,
+                           const unsigned long long* __restrict__ act, uint32_t rounds, const uint32_t* __restrict__ err) {
+    if (failed(err)) return;
+    uint32_t ran = 1;   // rounds that ran; the last one's output is the ranking
+    while (ran < rounds && round_runs(act, ran)) ++ran;
+    const RankRec* S = ran & 1 ? Sb : Sa;
     for (uint64_t x = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; x < n2; x += (uint64_t)gridDim.x * blockDim.x) {
         const uint2 nd = node[x];
         if (nd.y & SPLIT) {
@@ -352,7 +369,8 @@ __device__ __forceinline__ char oriented(const char* lab, uint32_t len, uint32_t
 // 3: per chain, once (by the lm-tig heading the list the host collator walks): flip the
 // list when its reverse complement starts with a smaller k-mer (ties keep the walk).
 __global__ void k_ut_flip(const uint32_t* __restrict__ lens, const char* const* __restrict__ label, uint64_t n,
-                          const RankRec* __restrict__ X, uint32_t k, uint8_t* flipb) {
+                          const RankRec* __restrict__ X, uint32_t k, uint8_t* flipb, const uint32_t* __restrict__ err) {
+    if (failed(err)) return;
     for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n; i += (uint64_t)gridDim.x * blockDim.x) {
         const uint32_t e0 = (uint32_t)(2 * i), e1 = e0 + 1;
         const RankRec x0 = X[e0], x1 = X[e1];
@@ -381,7 +399,9 @@ __global__ void k_ut_choose(const uint32_t* __restrict__ lens, const char* const
                             uint32_t* fin, unsigned long long* out_off, unsigned long long* cursor, unsigned long long* n_units,
                             unsigned long long* n_cyc, const uint32_t* __restrict__ job,
                             const unsigned long long* __restrict__ job_out_base, unsigned long long* job_cur,
-                            const uint8_t* __restrict__ flipb) {
+                            const uint8_t* __restrict__ flipb, const uint32_t* __restrict__ err, unsigned long long* err_out) {
+    if (blockIdx.x == 0 && threadIdx.x == 0) *err_out = *err;   // no later pass adds to it
+    if (failed(err)) return;
     const uint32_t lane = threadIdx.x & 31;
     const uint64_t stride = (uint64_t)gridDim.x * blockDim.x;
     for (uint64_t base = (uint64_t)blockIdx.x * blockDim.x; base < n; base += stride) {
@@ -729,7 +749,7 @@ bool UnitigBuffers::ensure(uint64_t n) {
     if (!b_label.ensure(8 * (n + 1)) || !b_tab.ensure(sizeof(EndSlot) * t) ||
         !b_partner.ensure(4 * n2) || !b_X0.ensure(sizeof(RankRec) * n2) || !b_X1.ensure(sizeof(RankRec) * n2) ||
         !b_fin.ensure(4 * (n + 1)) || !b_sx.ensure(4 * n2) || !b_sw.ensure(4 * n2) ||
-        !b_off.ensure(8 * n2) || !b_words.ensure(64) || !b_job.ensure(4 * (n + 1)) || !b_flip.ensure(n + 1) ||
+        !b_off.ensure(8 * n2) || !b_words.ensure(8 * (8 + MAX_ROUNDS)) || !h_words.ensure(64) || !b_job.ensure(4 * (n + 1)) || !b_flip.ensure(n + 1) ||
         !b_len.ensure(4 * (n + 1)) || !b_ends.ensure(16ull * end_words * (n + 1)))
         return false;
     len = b_len.as<uint32_t>();
@@ -823,10 +843,10 @@ int collate_device(const UnitigInput& in, UnitigBuffers& ub, cudaStream_t s, Uni
     const uint64_t n = in.n;
     ub.end_words = in.k > 63 ? 4 : 2;
     if (!ub.ensure(n)) return CFG_ERR_OOM;
-    if (cudaMemsetAsync(ub.words, 0, sizeof(unsigned long long) * 8, s) != cudaSuccess) return CFG_ERR_CUDA;
-    // [0] output bytes, [1] unitigs, [2] cycle lm-tigs, [3] active entries, [4] splitters,
-    // [5] insert tiles taken, [6] splitters taken by walks
-    unsigned long long* cursor = ub.words;
+    if (cudaMemsetAsync(ub.words, 0, sizeof(unsigned long long) * (8 + MAX_ROUNDS), s) != cudaSuccess) return CFG_ERR_CUDA;
+    // [0] output bytes, [1] unitigs, [2] cycle lm-tigs, [3] the error word, [4] splitters,
+    // [5] insert tiles taken, [6] splitters taken by walks, [8..] active entries after each round
+    unsigned long long *cursor = ub.words, *act = ub.words + 8;
     if (n == 0) return CFG_OK;
     if (2 * n >= SPLIT) return CFG_ERR_BAD_INPUT;   // entry ids are 31-bit
     const unsigned grid = 148 * 8;
@@ -852,36 +872,20 @@ int collate_device(const UnitigInput& in, UnitigBuffers& ub, cudaStream_t s, Uni
     RankRec* Sb[2] = {(RankRec*)ub.X[1], (RankRec*)ub.tab};   // the vertex table is done with
     k_rs_init<<<grid, 256, 0, s>>>(ub.len, n, ub.partner, in.k, 15u, node, ub.sx, ub.sw, cursor + 4, in.err);
     k_rs_walk<<<grid, 256, 0, s>>>(ub.sx, ub.sw, cursor + 4, node, Sb[0], cursor + 6, 4 * n + 64, in.err);
-    int cur = 0;
-    unsigned long long last = ~0ull;
-    for (int round = 0; round < 64; round += 2) {   // two rounds per look at the active count
-        k_ut_rank_round<<<grid, 256, 0, s>>>(cursor + 4, Sb[cur], Sb[cur ^ 1], nullptr);
-        cur ^= 1;
-        if (cudaMemsetAsync(cursor + 3, 0, 8, s) != cudaSuccess) return CFG_ERR_CUDA;
-        k_ut_rank_round<<<grid, 256, 0, s>>>(cursor + 4, Sb[cur], Sb[cur ^ 1], cursor + 3);
-        cur ^= 1;
-        res.rounds += 2;
-        unsigned long long active = 0;
-        if (cudaMemcpyAsync(&active, cursor + 3, 8, cudaMemcpyDeviceToHost, s) != cudaSuccess ||
-            cudaStreamSynchronize(s) != cudaSuccess)
-            return CFG_ERR_CUDA;
-        if (active == 0 || active == last) break;   // resolved, or only closed chains left
-        last = active;
-    }
-    // an invalid graph stops here, before any record is reserved or written
-    uint32_t e = 0;
-    if (cudaMemcpyAsync(&e, in.err, 4, cudaMemcpyDeviceToHost, s) != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess)
-        return CFG_ERR_CUDA;
-    if (e & DERR_BAD_GRAPH) return CFG_ERR_STATE;
-    if (e & DERR_WALK_LIMIT) return CFG_ERR_WALK_LIMIT;
-    k_rs_final<<<grid, 256, 0, s>>>(2 * n, node, X, Sb[cur]);
-    k_ut_flip<<<grid, 256, 0, s>>>(ub.len, ub.label, n, X, in.k, ub.flipb);
+    // a chain holds at most 2n splitters: this many rounds resolve every open one
+    uint32_t rounds = 1;
+    while (rounds < MAX_ROUNDS && (1ull << (rounds - 1)) < 2 * n) ++rounds;
+    for (uint32_t r = 0; r < rounds; ++r) k_ut_rank_round<<<grid, 256, 0, s>>>(cursor + 4, Sb[0], Sb[1], act, r, in.err);
+    k_rs_final<<<grid, 256, 0, s>>>(2 * n, node, X, Sb[0], Sb[1], act, rounds, in.err);
+    k_ut_flip<<<grid, 256, 0, s>>>(ub.len, ub.label, n, X, in.k, ub.flipb, in.err);
     k_ut_choose<<<grid, 256, 0, s>>>(ub.len, ub.label, n, ub.partner, X, in.k, ub.fin,
                                      ub.out_off, cursor, cursor + 1, cursor + 2, job, in.job_out_base, in.job_cur,
-                                     ub.flipb);
-    unsigned long long w[3] = {0, 0, 0};
-    if (cudaMemcpyAsync(w, cursor, 24, cudaMemcpyDeviceToHost, s) != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess)
+                                     ub.flipb, in.err, cursor + 3);
+    const unsigned long long* w = ub.h_words.as<unsigned long long>();
+    if (cudaMemcpyAsync(ub.h_words.p, cursor, 32, cudaMemcpyDeviceToHost, s) != cudaSuccess || cudaStreamSynchronize(s) != cudaSuccess)
         return CFG_ERR_CUDA;
+    if (w[3] & DERR_BAD_GRAPH) return CFG_ERR_STATE;
+    if (w[3] & DERR_WALK_LIMIT) return CFG_ERR_WALK_LIMIT;
     // a batch's output regions are sized by the caller before the call
     if (!in.jobs && !ub.ensure_out(w[0] + 16)) return CFG_ERR_OOM;
     k_ut_write<<<grid, 256, 0, s>>>(ub.len, ub.label, n, ub.fin, ub.partner, X, ub.out_off, in.k, ub.out);
