@@ -45,11 +45,12 @@ struct cfg_ctx {
     bool have_input = false, have_run = false;
 
     // partition
-    DevBuf flat, hist, misc, bucket_off, inst, fill, recs, scan_part, rcw;
+    DevBuf flat, words_d, bucket_off, inst, recs, scan_part, rcw;   // words_d: RunWords
+    HostBuf h_words;                                                 // its page-locked copy
     // plan
     DevBuf list, tab_off, tab_cap, arena;
     // outputs
-    DevBuf fasta, lm_text, lm, dump, retry, counters, stripe_cur, stripe_base, ut_lmbase, cyc_work, cyc_scratch, cyc_out;
+    DevBuf fasta, lm_text, lm, dump, retry, cyc_work, cyc_scratch, cyc_out;
     UnitigBuffers ub;
     HostBuf h_unitigs;
     uint64_t fasta_cap = 0, lm_text_cap = 0, lm_cap = 0, dump_cap = 0;   // per output stripe
@@ -89,11 +90,15 @@ uint32_t next_pow2(uint64_t v) {
     return (uint32_t)std::min<uint64_t>(p, 1ull << 31);
 }
 
-struct MiscWords {   // small device-side words, one allocation
-    unsigned long long rec_cursor;
-    uint32_t err;
-    uint32_t pad;
-};
+RunWords* dev_words(cfg_ctx* c) { return c->words_d.as<RunWords>(); }
+const RunWords* host_words(cfg_ctx* c) { return c->h_words.as<RunWords>(); }
+
+// The run's device words to the host, and waits for them (and all work before them).
+int read_words(cfg_ctx* c) {
+    CK(cudaMemcpyAsync(c->h_words.p, c->words_d.p, sizeof(RunWords), cudaMemcpyDeviceToHost, c->stream));
+    CK(cudaStreamSynchronize(c->stream));
+    return CFG_OK;
+}
 
 int check_err_word(cfg_ctx* c, uint32_t e) {
     if (e & DERR_MISSING_KEY) return fail(c, CFG_ERR_WALK_LIMIT, "neighbour k-mer missing from its subgraph table");
@@ -102,12 +107,35 @@ int check_err_word(cfg_ctx* c, uint32_t e) {
     return CFG_OK;
 }
 
-// Partition + bucket scatter.  Leaves bucketed records in c->recs and per-subgraph
-// instance counts in `inst_h`.
-int run_partition(cfg_ctx* c, std::vector<uint32_t>& inst_h, std::vector<uint32_t>& off_h) {
+// The subgraphs' table shapes and launch order, planned on the device from `inst`.
+PlanArgs plan_args(cfg_ctx* c) {
+    PlanArgs a{};
+    a.inst = c->inst.as<uint32_t>(); a.G = c->G; a.words = c->words;
+    // expected distinct vertices per k-mer instance, in percent; tables are sized for
+    // a load factor near one half of that estimate
+    a.load = c->p.table_load_pct ? c->p.table_load_pct : 100;
+    const LocalShape* sh = local_shapes(c->words, a.n_shapes);
+    for (uint32_t i = 0; i < a.n_shapes; ++i) a.slots[i] = sh[i].slots;
+    a.per_cl = subgraph_cluster_per_cta(c->words);
+    // k <= 31: clusters of up to 8 CTAs beat arena tables in HBM; k > 32 (24-byte key and
+    // state) the L2-resident arena tables win
+    a.max_cluster = c->words == 1 ? 8 : 1;
+    a.list = c->list.as<uint32_t>(); a.tab_off = c->tab_off.as<uint64_t>(); a.tab_cap = c->tab_cap.as<uint32_t>();
+    a.w = dev_words(c);
+    return a;
+}
+
+// Partition, bucket sort and plan, queued together and waited for once.  Leaves bucketed
+// records in c->recs, per-subgraph instance counts in c->inst, the launch lists, and the
+// run's words on the host.
+int run_partition(cfg_ctx* c) {
     const uint32_t G = c->G;
-    if (!c->misc.ensure(sizeof(MiscWords))) return fail(c, CFG_ERR_OOM, "misc");
     uint64_t cap = std::max<uint64_t>(c->n_bases / 4 + 1024, 1u << 16);
+    if (!c->words_d.ensure(sizeof(RunWords)) || !c->h_words.ensure(sizeof(RunWords))) return fail(c, CFG_ERR_OOM, "run words");
+    if (!c->bucket_off.ensure(4ull * (G + 1)) || !c->inst.ensure(4ull * G) || !c->list.ensure(4ull * G) ||
+        !c->tab_off.ensure(8ull * G) || !c->tab_cap.ensure(4ull * G))
+        return fail(c, CFG_ERR_OOM, "bucket arrays");
+    if (!c->scan_part.ensure(4ull * bucket_sort_scratch_words(G, c->sms))) return fail(c, CFG_ERR_OOM, "sort scratch");
     for (int attempt = 0; attempt < 3; ++attempt) {
         {   // the partition's records and the bucket sort's: equal capacities, because the two
             // buffers trade places after every sort (and neither may be reallocated after the
@@ -117,16 +145,16 @@ int run_partition(cfg_ctx* c, std::vector<uint32_t>& inst_h, std::vector<uint32_
             if (!c->flat.ensure_exact(want) || !c->recs.ensure_exact(want)) return fail(c, CFG_ERR_OOM, "record buffers");
         }
         cap = std::min(c->flat.bytes, c->recs.bytes) / 8;
-        CK(cudaMemsetAsync(c->misc.p, 0, sizeof(MiscWords), c->stream));
+        CK(cudaMemsetAsync(c->words_d.p, 0, sizeof(RunWords), c->stream));
         PartitionArgs a{};
         a.packed = c->d_packed; a.frag_off = c->d_frag_off; a.frag_len = c->d_frag_len;
         a.n_frags = c->n_frags; a.n_bases = c->n_bases;
         a.k = c->p.k; a.l = c->p.l; a.w = c->p.k - c->p.l;
         a.gmask = G - 1; a.seed0 = wy_seed0_host(); a.seg = partition_segment(c->n_bases, a.w);
         a.recs = c->flat.as<uint64_t>(); a.rec_cap = cap;
-        a.rec_cursor = &c->misc.as<MiscWords>()->rec_cursor;
+        a.rec_cursor = &dev_words(c)->rec_cursor;
         a.hist = nullptr;   // the bucket sort counts records and instances per subgraph
-        a.err = &c->misc.as<MiscWords>()->err;
+        a.err = &dev_words(c)->err;
         const uint64_t n_words = (c->n_bases + 31) / 32;
         if (!c->rcw.ensure(8 * (n_words + 4))) return fail(c, CFG_ERR_OOM, "reverse-complement words");
         a.rcw = c->rcw.as<uint64_t>();
@@ -154,81 +182,128 @@ int run_partition(cfg_ctx* c, std::vector<uint32_t>& inst_h, std::vector<uint32_
         }
         CK(cudaGetLastError());
         CK(cudaEventRecord(c->ev[2], c->stream));
-        MiscWords m{};
-        CK(cudaMemcpyAsync(&m, c->misc.p, sizeof(m), cudaMemcpyDeviceToHost, c->stream));
-        CK(cudaStreamSynchronize(c->stream));
-        if (m.err & DERR_BAD_FRAG)
+        CK(cudaEventRecord(c->ev[3], c->stream));
+        // flat -> recs (by super-bucket) -> flat (by subgraph), then the two buffers trade
+        // places: c->recs holds the bucketed records, c->flat the next run's partition output
+        CK(launch_bucket_sort(c->flat.as<uint64_t>(), a.rec_cursor, cap, G, c->p.k, c->sms, c->scan_part.as<uint32_t>(),
+                              c->recs.as<uint64_t>(), c->flat.as<uint64_t>(), c->bucket_off.as<uint32_t>(),
+                              c->inst.as<uint32_t>(), c->stream));
+        CK(cudaEventRecord(c->ev[4], c->stream));
+        launch_run_plan(plan_args(c), c->stream);
+        CK(cudaGetLastError());
+        c->launches += 7;
+        const int rc = read_words(c);
+        if (rc) return rc;
+        const RunWords& w = *host_words(c);
+        if (w.err & DERR_BAD_FRAG)
             return fail(c, CFG_ERR_BAD_INPUT, "a fragment runs past n_bases or holds fewer than k+1 bases");
-        if (m.rec_cursor <= cap && !(m.err & DERR_REC_OVERFLOW)) { c->n_records = m.rec_cursor; break; }
-        cap = m.rec_cursor + 1024;
-        if (attempt == 2) return fail(c, CFG_ERR_OOM, "record buffer kept overflowing");
+        if (w.rec_cursor <= cap && !(w.err & DERR_REC_OVERFLOW)) {
+            std::swap(c->flat, c->recs);
+            c->n_records = w.rec_cursor;
+            c->n_instances = w.instances;
+            return CFG_OK;
+        }
+        cap = w.rec_cursor + 1024;
     }
-    CK(cudaEventRecord(c->ev[3], c->stream));
-    if (!c->bucket_off.ensure(4ull * (G + 1)) || !c->inst.ensure(4ull * G)) return fail(c, CFG_ERR_OOM, "bucket arrays");
-    // flat -> recs (by super-bucket) -> flat (by subgraph), then the two buffers trade
-    // places: c->recs holds the bucketed records, c->flat the next run's partition output
-    if (!c->scan_part.ensure(4ull * bucket_sort_scratch_words(G, c->sms))) return fail(c, CFG_ERR_OOM, "sort scratch");
-    CK(launch_bucket_sort(c->flat.as<uint64_t>(), c->n_records, G, c->p.k, c->sms, c->scan_part.as<uint32_t>(),
-                          c->recs.as<uint64_t>(), c->flat.as<uint64_t>(), c->bucket_off.as<uint32_t>(),
-                          c->inst.as<uint32_t>(), c->stream));
-    std::swap(c->flat, c->recs);
-    CK(cudaEventRecord(c->ev[4], c->stream));
-    c->launches += 5;
-    inst_h.resize(G); off_h.resize(G + 1);
-    CK(cudaMemcpyAsync(inst_h.data(), c->inst.p, 4ull * G, cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaMemcpyAsync(off_h.data(), c->bucket_off.p, 4ull * (G + 1), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    c->n_instances = 0;
-    for (uint32_t g = 0; g < G; ++g) c->n_instances += inst_h[g];
+    return fail(c, CFG_ERR_OOM, "record buffer kept overflowing");
+}
+
+// One launch: n subgraphs sharing a table shape (cluster 0: arena tables, with their offsets
+// and capacities; else `cluster` CTAs with `per` slots each), listed at `at` of the plan arrays.
+struct Launch { uint32_t at = 0, n = 0, per = 0, cluster = 0, threads = 0; };
+
+int launch_one(cfg_ctx* c, const Launch& L) {
+    const int W = c->words;
+    SubgraphArgs a{};
+    a.packed = c->d_packed; a.recs = c->recs.as<uint64_t>(); a.bucket_off = c->bucket_off.as<uint32_t>();
+    a.list = c->list.as<uint32_t>() + L.at; a.n_list = L.n;
+    a.tab_off = c->tab_off.as<uint64_t>() + L.at; a.tab_cap = c->tab_cap.as<uint32_t>() + L.at;
+    a.smem_cap = L.per; a.arena = c->arena.as<unsigned char>();
+    a.k = c->p.k; a.fth = c->p.cutoff; a.load_limit_pct = 90; a.record_clocks = 1;
+    a.dedup = record_dedup(c->p.k, c->p.l, c->p.cutoff, c->p.flags);
+    a.fasta = c->fasta.as<char>(); a.fasta_cap = c->fasta_cap;
+    a.lm_text = c->lm_text.as<char>(); a.lm_text_cap = c->lm_text_cap;
+    a.lm = c->lm.as<LmtigOut>(); a.lm_cap = c->lm_cap;
+    a.stripe_cur = dev_words(c)->stripe_cur; a.stripes = c->stripes;
+    a.dump = (c->p.flags & CFG_FLAG_DUMP_STATES) ? c->dump.as<StateOut>() : nullptr; a.dump_cap = c->dump_cap;
+    a.retry = c->retry.as<uint32_t>(); a.cnt = &dev_words(c)->cnt;
+    a.err = &dev_words(c)->err;
+    // the table shape's threads, unless the caller set slots per thread; clusters and arena
+    // tables: a quarter of the slots, or the largest CTA
+    const uint32_t tmax = subgraph_max_threads(W, L.cluster == 0 ? 0u : L.per), div = c->p.slots_per_thread;
+    const uint32_t threads = L.cluster == 0 ? tmax
+                             : L.cluster == 1 && !div ? L.threads
+                             : L.cluster == 1 && L.per > 4096 ? tmax
+                             : std::min<uint32_t>(tmax, (std::max<uint32_t>(64, L.per / (div ? div : 4)) + 31) / 32 * 32);
+    CK(launch_subgraphs(a, W, L.cluster, threads, c->stream));
+    c->launches += 1;
     return CFG_OK;
 }
 
-// One launch: subgraphs sharing a table shape.  cluster 0 = global arena tables
-// (per-entry offset/capacity), else `cluster` CTAs with `per` slots each.
-struct Launch { std::vector<uint32_t> list; std::vector<uint64_t> off; std::vector<uint32_t> cap; uint32_t per = 0; uint32_t cluster = 0; uint32_t threads = 0; };
+int ensure_arena(cfg_ctx* c, uint64_t slots) {
+    if (slots && !c->arena.ensure(slots * slot_bytes(c->words))) return fail(c, CFG_ERR_OOM, "table arena");
+    return CFG_OK;
+}
 
-int launch_plan(cfg_ctx* c, const std::vector<Launch>& plan, uint64_t arena_slots) {
-    const int W = c->words;
-    if (arena_slots && !c->arena.ensure(arena_slots * slot_bytes(W))) return fail(c, CFG_ERR_OOM, "table arena");
-    size_t n_total = 0;
-    for (const Launch& L : plan) n_total += L.list.size();
-    if (!c->list.ensure(4 * std::max<size_t>(n_total, 1)) || !c->tab_off.ensure(8 * std::max<size_t>(n_total, 1)) ||
-        !c->tab_cap.ensure(4 * std::max<size_t>(n_total, 1)))
-        return fail(c, CFG_ERR_OOM, "plan arrays");
-    size_t at = 0;
-    for (const Launch& L : plan) {
-        if (L.list.empty()) continue;
-        uint32_t* d_list = c->list.as<uint32_t>() + at;
-        uint64_t* d_off = c->tab_off.as<uint64_t>() + at;
-        uint32_t* d_cap = c->tab_cap.as<uint32_t>() + at;
-        CK(cudaMemcpyAsync(d_list, L.list.data(), 4 * L.list.size(), cudaMemcpyHostToDevice, c->stream));
-        if (L.cluster == 0) {
-            CK(cudaMemcpyAsync(d_off, L.off.data(), 8 * L.off.size(), cudaMemcpyHostToDevice, c->stream));
-            CK(cudaMemcpyAsync(d_cap, L.cap.data(), 4 * L.cap.size(), cudaMemcpyHostToDevice, c->stream));
+// Every subgraph once, as planned on the device.
+int launch_planned(cfg_ctx* c, const RunWords& w) {
+    const PlanArgs pa = plan_args(c);
+    int rc = ensure_arena(c, w.arena_slots);
+    if (rc) return rc;
+    uint32_t n_shapes = 0;
+    const LocalShape* shapes = local_shapes(c->words, n_shapes);
+    Launch L;
+    for (uint32_t cls = 0; cls < 8 + pa.n_shapes; ++cls, L.at += L.n) {
+        L.n = 0;
+        for (uint32_t b = 0; b < PLAN_SUB; ++b) L.n += w.bins[cls * PLAN_SUB + b];
+        if (!L.n) continue;
+        L.cluster = cls == 0 ? 0 : cls < 8 ? 9 - cls : 1;
+        const LocalShape* sh = cls < 8 ? nullptr : &shapes[n_shapes - 1 - (cls - 8)];
+        L.per = sh ? sh->slots : pa.per_cl;
+        L.threads = sh ? sh->threads : 0;
+        rc = launch_one(c, L);
+        if (rc) return rc;
+    }
+    return CFG_OK;
+}
+
+// The subgraphs in `work` again, with tables for want[i] slots.
+int launch_retries(cfg_ctx* c, const std::vector<uint32_t>& work, const std::vector<uint64_t>& want) {
+    const PlanArgs pa = plan_args(c);
+    uint32_t n_shapes = 0;
+    const LocalShape* shapes = local_shapes(c->words, n_shapes);
+    std::vector<std::vector<uint32_t>> of(9 + n_shapes);   // arena, clusters of 1..8, one-CTA shapes
+    std::vector<uint64_t> off;
+    std::vector<uint32_t> cap;
+    uint64_t arena_slots = 0;
+    for (size_t i = 0; i < work.size(); ++i) {
+        const uint64_t w = want[i], fit = local_fit(c->words, w);
+        uint32_t sh = 0;
+        while (sh < n_shapes && shapes[sh].slots < fit) ++sh;
+        if (sh < n_shapes) of[9 + sh].push_back(work[i]);
+        else if (w <= (uint64_t)pa.per_cl * pa.max_cluster) of[(w + pa.per_cl - 1) / pa.per_cl].push_back(work[i]);
+        else {
+            of[0].push_back(work[i]);
+            off.push_back(arena_slots); cap.push_back(next_pow2(w));
+            arena_slots += cap.back();
         }
-        SubgraphArgs a{};
-        a.packed = c->d_packed; a.recs = c->recs.as<uint64_t>(); a.bucket_off = c->bucket_off.as<uint32_t>();
-        a.list = d_list; a.n_list = (uint32_t)L.list.size();
-        a.tab_off = d_off; a.tab_cap = d_cap; a.smem_cap = L.per; a.arena = c->arena.as<unsigned char>();
-        a.k = c->p.k; a.fth = c->p.cutoff; a.load_limit_pct = 90; a.record_clocks = 1;
-        a.dedup = record_dedup(c->p.k, c->p.l, c->p.cutoff, c->p.flags);
-        a.fasta = c->fasta.as<char>(); a.fasta_cap = c->fasta_cap;
-        a.lm_text = c->lm_text.as<char>(); a.lm_text_cap = c->lm_text_cap;
-        a.lm = c->lm.as<LmtigOut>(); a.lm_cap = c->lm_cap;
-        a.stripe_cur = c->stripe_cur.as<unsigned long long>(); a.stripes = c->stripes;
-        a.dump = (c->p.flags & CFG_FLAG_DUMP_STATES) ? c->dump.as<StateOut>() : nullptr; a.dump_cap = c->dump_cap;
-        a.retry = c->retry.as<uint32_t>(); a.cnt = c->counters.as<Counters>();
-        a.err = &c->misc.as<MiscWords>()->err;
-        // the table shape's threads, unless the caller set slots per thread; clusters and arena
-        // tables: a quarter of the slots, or the largest CTA
-        const uint32_t tmax = subgraph_max_threads(W, L.cluster == 0 ? 0u : L.per), div = c->p.slots_per_thread;
-        const uint32_t threads = L.cluster == 0 ? tmax
-                                 : L.cluster == 1 && !div ? L.threads
-                                 : L.cluster == 1 && L.per > 4096 ? tmax
-                                 : std::min<uint32_t>(tmax, (std::max<uint32_t>(64, L.per / (div ? div : 4)) + 31) / 32 * 32);
-        CK(launch_subgraphs(a, W, L.cluster, threads, c->stream));
-        c->launches += 1;
-        at += L.list.size();
+    }
+    int rc = ensure_arena(c, arena_slots);
+    if (rc) return rc;
+    if (!off.empty()) {
+        CK(cudaMemcpyAsync(c->tab_off.p, off.data(), 8 * off.size(), cudaMemcpyHostToDevice, c->stream));
+        CK(cudaMemcpyAsync(c->tab_cap.p, cap.data(), 4 * cap.size(), cudaMemcpyHostToDevice, c->stream));
+    }
+    Launch L;
+    for (uint32_t s = 0; s < of.size(); ++s, L.at += L.n) {
+        L.n = (uint32_t)of[s].size();
+        if (!L.n) continue;
+        CK(cudaMemcpyAsync(c->list.as<uint32_t>() + L.at, of[s].data(), 4ull * L.n, cudaMemcpyHostToDevice, c->stream));
+        L.cluster = s == 0 ? 0 : s < 9 ? s : 1;
+        L.per = s < 9 ? pa.per_cl : shapes[s - 9].slots;
+        L.threads = s < 9 ? 0 : shapes[s - 9].threads;
+        rc = launch_one(c, L);
+        if (rc) return rc;
     }
     return CFG_OK;
 }
@@ -244,10 +319,7 @@ int ensure_outputs(cfg_ctx* c, uint64_t fasta_need, uint64_t lm_text_need, uint6
     c->lm_text_cap = c->lm_text.bytes / S;
     if (!c->lm.ensure(S * slice(lm_need) * sizeof(LmtigOut))) return fail(c, CFG_ERR_OOM, "lm-tig records");
     c->lm_cap = c->lm.bytes / sizeof(LmtigOut) / S;
-    if (!c->stripe_cur.ensure(8ull * JOB_CUR_STRIDE * OUT_STRIPES) || !c->stripe_base.ensure(8ull * OUT_STRIPES))
-        return fail(c, CFG_ERR_OOM, "stripe cursors");
     if (!c->retry.ensure(4ull * c->G)) return fail(c, CFG_ERR_OOM, "retry list");
-    if (!c->counters.ensure(sizeof(Counters))) return fail(c, CFG_ERR_OOM, "counters");
     if (c->p.flags & CFG_FLAG_DUMP_STATES) {
         if (!c->dump.ensure(sizeof(StateOut) * std::max<uint64_t>(c->n_instances, 1))) return fail(c, CFG_ERR_OOM, "state dump");
         c->dump_cap = c->dump.bytes / sizeof(StateOut);
@@ -255,96 +327,47 @@ int ensure_outputs(cfg_ctx* c, uint64_t fasta_need, uint64_t lm_text_need, uint6
     return CFG_OK;
 }
 
-int run_subgraphs(cfg_ctx* c, const std::vector<uint32_t>& inst_h) {
-    const uint32_t G = c->G;
-    const int W = c->words;
-    // expected distinct vertices per k-mer instance, in percent; tables are sized for
-    // a load factor near one half of that estimate
-    const uint32_t load = c->p.table_load_pct ? c->p.table_load_pct : 100;
-    uint32_t n_shapes = 0;
-    const LocalShape* shapes = local_shapes(W, n_shapes);   // one CTA's table
-    const uint32_t per_cl = subgraph_cluster_per_cta(W);   // each CTA of a cluster
-    // k <= 31: clusters of up to 8 CTAs beat arena tables in HBM; k > 32 (24-byte key and
-    // state, 128-register kernels, one CTA per SM) the L2-resident arena tables win
-    const uint32_t max_cluster = W == 1 ? 8 : 1;
-    std::vector<uint64_t> want(G, 0);                      // slots wanted per subgraph
-    for (uint32_t g = 0; g < G; ++g)
-        if (inst_h[g]) want[g] = std::max<uint64_t>(64, ((uint64_t)inst_h[g] * load * 2 + 99) / 100);
+int run_subgraphs(cfg_ctx* c) {
+    const RunWords& w = *host_words(c);   // from run_partition, then from each pass
     uint64_t fasta_need = c->n_bases + (c->n_records + 1024) * 8 + (1u << 20);
     // lm-tig labels: at most every k-mer instance once plus k-1 bases per lm-tig, and the
     // records' lengths sum to at most n_bases + k per record
     uint64_t lm_text_need = c->n_bases + (c->n_records + 1024) * (c->p.k + 1);
     uint64_t lm_need = c->n_records + 1024;
-    // larger subgraphs first (src/Subgraphs_Manager.cpp:222-231): a counting sort on a
-    // log-scale size key (eight steps per doubling), enough to start the big ones early
-    std::vector<uint32_t> todo;
-    {
-        auto key = [](uint32_t n) -> uint32_t {   // 8 * log2(n), in [0, 255]
-            const uint32_t e = 31 - __builtin_clz(n);
-            const uint32_t frac = e >= 3 ? (n >> (e - 3)) & 7 : (n << (3 - e)) & 7;
-            return 8 * e + frac;
-        };
-        uint32_t cnt[257] = {0};
-        for (uint32_t g = 0; g < G; ++g) if (inst_h[g]) ++cnt[255 - key(inst_h[g]) + 1];
-        for (uint32_t b = 1; b < 257; ++b) cnt[b] += cnt[b - 1];
-        todo.resize(cnt[256]);
-        for (uint32_t g = 0; g < G; ++g) if (inst_h[g]) todo[cnt[255 - key(inst_h[g])]++] = g;
-    }
-
     for (int round = 0; round < 3; ++round) {   // output-arena overflow: regrow, rerun all
         int rc = ensure_outputs(c, fasta_need, lm_text_need, lm_need);
         if (rc) return rc;
-        CK(cudaMemsetAsync(c->counters.p, 0, sizeof(Counters), c->stream));
-        CK(cudaMemsetAsync(c->stripe_cur.p, 0, 8ull * JOB_CUR_STRIDE * OUT_STRIPES, c->stream));
-        std::vector<uint32_t> work = todo;
-        std::vector<uint64_t> cur_want = want;
+        if (round) {   // the counters and cursors start over, and so does the list (a pass of retries may have overwritten it)
+            CK(cudaMemsetAsync(c->words_d.p, 0, sizeof(RunWords), c->stream));
+            launch_run_plan(plan_args(c), c->stream);
+            CK(cudaGetLastError());
+            rc = read_words(c);
+            if (rc) return rc;
+        }
+        std::vector<uint32_t> work;
+        std::vector<uint64_t> want;      // slots of each subgraph in `work`
+        std::vector<uint64_t> grown;     // per subgraph, once one is retried: its slots so far
         uint64_t retries = 0;
         bool overflow = false;
-        for (int pass = 0; pass < 12 && !work.empty(); ++pass) {
-            std::vector<Launch> plan;
-            int shape_at[16 + 9];   // launch of each one-CTA shape, then of each cluster size
-            std::fill(shape_at, shape_at + 16 + 9, -1);
-            Launch glob; glob.cluster = 0;
-            uint64_t arena_slots = 0;
-            for (uint32_t g : work) {
-                const uint64_t w = cur_want[g];
-                uint32_t cl, per, sh = 0;
-                const uint64_t fit = local_fit(W, w);
-                while (sh < n_shapes && shapes[sh].slots < fit) ++sh;
-                if (sh < n_shapes) { cl = 1; per = shapes[sh].slots; }
-                else if (w <= (uint64_t)per_cl * max_cluster) { cl = (uint32_t)((w + per_cl - 1) / per_cl); per = per_cl; }
-                else {
-                    const uint32_t cap = next_pow2(w);
-                    glob.list.push_back(g); glob.off.push_back(arena_slots); glob.cap.push_back(cap);
-                    arena_slots += cap;
-                    continue;
-                }
-                // one launch per shape
-                const uint32_t sk = cl == 1 ? sh : 16 + cl;
-                if (shape_at[sk] < 0) {
-                    shape_at[sk] = (int)plan.size();
-                    plan.emplace_back(); plan.back().per = per; plan.back().cluster = cl;
-                    plan.back().threads = cl == 1 ? shapes[sh].threads : 0;
-                }
-                plan[shape_at[sk]].list.push_back(g);
-            }
-            plan.push_back(glob);
-            CK(cudaMemsetAsync(&c->counters.as<Counters>()->retry_count, 0, sizeof(unsigned long long), c->stream));
+        for (int pass = 0; pass < 12 && (pass == 0 || !work.empty()); ++pass) {
             CK(cudaEventRecord(c->ev[5], c->stream));
-            rc = launch_plan(c, plan, arena_slots);
+            if (pass == 0) rc = launch_planned(c, w);
+            else {
+                CK(cudaMemsetAsync(&dev_words(c)->cnt.retry_count, 0, sizeof(unsigned long long), c->stream));
+                rc = launch_retries(c, work, want);
+            }
             if (rc) return rc;
             CK(cudaEventRecord(c->ev[6], c->stream));
-            Counters h{};
-            MiscWords m{};
-            unsigned long long cur[JOB_CUR_STRIDE * OUT_STRIPES];
-            CK(cudaMemcpyAsync(&h, c->counters.p, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
-            CK(cudaMemcpyAsync(&m, c->misc.p, sizeof(m), cudaMemcpyDeviceToHost, c->stream));
-            CK(cudaMemcpyAsync(cur, c->stripe_cur.p, sizeof(cur), cudaMemcpyDeviceToHost, c->stream));
-            CK(cudaStreamSynchronize(c->stream));
+            launch_stripe_fixup(c->lm.as<LmtigOut>(), c->lm_cap, dev_words(c), c->stream);
+            CK(cudaGetLastError());
+            c->launches += 1;
+            CK(cudaEventRecord(c->ev[7], c->stream));
+            rc = read_words(c);
+            if (rc) return rc;
             uint64_t max_f = 0, max_t = 0, max_l = 0;
             for (uint32_t st = 0; st < OUT_STRIPES; ++st) {
-                c->s_fasta[st] = cur[st * JOB_CUR_STRIDE]; c->s_text[st] = cur[st * JOB_CUR_STRIDE + 1];
-                c->s_lm[st] = cur[st * JOB_CUR_STRIDE + 2];
+                c->s_fasta[st] = w.stripe_cur[st * JOB_CUR_STRIDE]; c->s_text[st] = w.stripe_cur[st * JOB_CUR_STRIDE + 1];
+                c->s_lm[st] = w.stripe_cur[st * JOB_CUR_STRIDE + 2];
                 max_f = std::max<uint64_t>(max_f, c->s_fasta[st]); max_t = std::max<uint64_t>(max_t, c->s_text[st]);
                 max_l = std::max<uint64_t>(max_l, c->s_lm[st]);
             }
@@ -353,47 +376,44 @@ int run_subgraphs(cfg_ctx* c, const std::vector<uint32_t>& inst_h) {
                 cudaEventElapsedTime(&ms, c->ev[5], c->ev[6]);
                 c->sub_ms += ms;
             }
-            rc = check_err_word(c, m.err);
+            rc = check_err_word(c, w.err);
             if (rc) return rc;
-            if (m.err & (DERR_OUT_OVERFLOW | DERR_DUMP_OVERFLOW)) {
+            if (w.err & (DERR_OUT_OVERFLOW | DERR_DUMP_OVERFLOW)) {
                 fasta_need = std::max<uint64_t>(fasta_need, max_f * c->stripes) * 2;
                 lm_text_need = std::max<uint64_t>(lm_text_need, max_t * c->stripes) * 2;
                 lm_need = std::max<uint64_t>(lm_need, max_l * c->stripes) * 2;
-                CK(cudaMemsetAsync(&c->misc.as<MiscWords>()->err, 0, sizeof(uint32_t), c->stream));
                 overflow = true;
                 break;
             }
-            work.clear();
-            if (h.retry_count) {
-                work.resize(h.retry_count);
-                CK(cudaMemcpyAsync(work.data(), c->retry.p, 4 * h.retry_count, cudaMemcpyDeviceToHost, c->stream));
-                CK(cudaStreamSynchronize(c->stream));
-                retries += h.retry_count;
-                for (uint32_t g : work) {
-                    if (cur_want[g] >= (1ull << 30)) return fail(c, CFG_ERR_TABLE_FULL, "subgraph table exceeded 2^30 slots");
-                    cur_want[g] *= 4;
+            const uint64_t n_retry = w.cnt.retry_count;
+            work.resize(n_retry);
+            want.resize(n_retry);
+            if (n_retry) {
+                CK(cudaMemcpyAsync(work.data(), c->retry.p, 4 * n_retry, cudaMemcpyDeviceToHost, c->stream));
+                if (grown.empty()) {   // rare: a plan from the instance counts on the host
+                    std::vector<uint32_t> inst(c->G);
+                    CK(cudaMemcpyAsync(inst.data(), c->inst.p, 4ull * c->G, cudaMemcpyDeviceToHost, c->stream));
+                    CK(cudaStreamSynchronize(c->stream));
+                    const uint32_t load = plan_args(c).load;
+                    grown.resize(c->G);
+                    for (uint32_t g = 0; g < c->G; ++g) grown[g] = std::max<uint64_t>(64, ((uint64_t)inst[g] * load * 2 + 99) / 100);
+                } else {
+                    CK(cudaStreamSynchronize(c->stream));
+                }
+                retries += n_retry;
+                for (size_t i = 0; i < work.size(); ++i) {
+                    uint64_t& x = grown[work[i]];
+                    if (x >= (1ull << 30)) return fail(c, CFG_ERR_TABLE_FULL, "subgraph table exceeded 2^30 slots");
+                    x *= 4;
+                    want[i] = x;
                 }
             }
         }
         if (overflow) continue;
         if (!work.empty()) return fail(c, CFG_ERR_TABLE_FULL, "subgraph tables kept overflowing");
-        Counters h{};
-        CK(cudaMemcpyAsync(&h, c->counters.p, sizeof(h), cudaMemcpyDeviceToHost, c->stream));
-        CK(cudaStreamSynchronize(c->stream));
-        // label offsets of each stripe's lm-tigs become offsets into the joined label text
         uint64_t fb = 0, tb = 0, nl = 0;
-        unsigned long long base[OUT_STRIPES];
-        for (uint32_t st = 0; st < OUT_STRIPES; ++st) {
-            base[st] = tb;
-            fb += c->s_fasta[st]; tb += c->s_text[st]; nl += c->s_lm[st];
-        }
-        if (nl) {
-            CK(cudaMemcpyAsync(c->stripe_base.p, base, sizeof(base), cudaMemcpyHostToDevice, c->stream));
-            launch_stripe_fixup(c->lm.as<LmtigOut>(), c->lm_cap, c->stripe_cur.as<unsigned long long>(),
-                                c->stripe_base.as<unsigned long long>(), OUT_STRIPES, c->stream);
-            CK(cudaGetLastError());
-            c->launches += 1;
-        }
+        for (uint32_t st = 0; st < OUT_STRIPES; ++st) { fb += c->s_fasta[st]; tb += c->s_text[st]; nl += c->s_lm[st]; }
+        const Counters& h = w.cnt;
         cfg_counts& o = c->counts;
         o.n_bases = c->n_bases; o.n_records = c->n_records; o.n_instances = c->n_instances;
         o.n_vertices = h.vertices; o.n_isolated = h.isolated; o.n_phantom = h.phantom;
@@ -603,13 +623,10 @@ int cfg_run(cfg_ctx* c) {
     c->sub_ms = 0;
     c->launches = 0;
     CK(cudaEventRecord(c->ev[0], c->stream));
-    std::vector<uint32_t> inst_h, off_h;
-    int rc = run_partition(c, inst_h, off_h);
+    int rc = run_partition(c);
     if (rc) return rc;
-    rc = run_subgraphs(c, inst_h);
+    rc = run_subgraphs(c);   // waits for its last pass, whose end is ev[7]
     if (rc) return rc;
-    CK(cudaEventRecord(c->ev[7], c->stream));
-    CK(cudaEventSynchronize(c->ev[7]));
     float tp = 0, ts = 0, tt = 0;
     cudaEventElapsedTime(&tp, c->ev[1], c->ev[2]);
     cudaEventElapsedTime(&ts, c->ev[3], c->ev[4]);
@@ -696,39 +713,32 @@ int cfg_unitigs(cfg_ctx* c, const char** fasta, uint64_t* bytes, uint64_t* n_uni
     if (!c->have_run) return fail(c, CFG_ERR_STATE, "no completed run");
     CK(cudaSetDevice(c->device));
     const cfg_counts& n = c->counts;
-    unsigned long long lb[OUT_STRIPES], acc = 0;
-    for (uint32_t st = 0; st < OUT_STRIPES; ++st) { lb[st] = acc; acc += c->s_lm[st]; }
-    if (!c->ut_lmbase.ensure(sizeof(lb)) || !c->cyc_out.ensure(16)) return fail(c, CFG_ERR_OOM, "collation buffers");
-    CK(cudaMemcpyAsync(c->ut_lmbase.p, lb, sizeof(lb), cudaMemcpyHostToDevice, c->stream));
-    CK(cudaMemsetAsync(&c->misc.as<MiscWords>()->err, 0, sizeof(uint32_t), c->stream));
+    if (!c->cyc_out.ensure(16)) return fail(c, CFG_ERR_OOM, "collation buffers");
+    CK(cudaMemsetAsync(&dev_words(c)->err, 0, sizeof(uint32_t), c->stream));
     CK(cudaEventRecord(c->ev[0], c->stream));
     UnitigInput in{};
     in.lm = c->lm.as<LmtigOut>(); in.lm_slice = c->lm_cap;
     in.text = c->lm_text.as<char>(); in.text_slice = c->lm_text_cap;
-    in.stripe_cur = c->stripe_cur.as<unsigned long long>();
-    in.lm_base = c->ut_lmbase.as<unsigned long long>(); in.text_base = c->stripe_base.as<unsigned long long>();
-    in.stripes = c->stripes; in.k = c->p.k; in.n = n.n_lmtig; in.err = &c->misc.as<MiscWords>()->err;
+    in.stripe_cur = dev_words(c)->stripe_cur;
+    in.lm_base = dev_words(c)->lm_base; in.text_base = dev_words(c)->text_base;
+    in.stripes = c->stripes; in.k = c->p.k; in.n = n.n_lmtig; in.err = &dev_words(c)->err;
     UnitigResult res{};
     int rc = collate_device(in, c->ub, c->stream, res);
     if (rc == CFG_ERR_OOM) return fail(c, rc, "collation buffers");
     if (rc == CFG_ERR_STATE) return fail(c, rc, "lm-tig ends do not form a valid discontinuity graph");
     if (rc == CFG_ERR_WALK_LIMIT) return fail(c, rc, "lm-tig ranking exceeded its bound");
     if (rc) return fail(c, rc, std::string("collation: ") + cudaGetErrorString(cudaGetLastError()));
-    MiscWords m{};
-    CK(cudaMemcpyAsync(&m, c->misc.p, sizeof(m), cudaMemcpyDeviceToHost, c->stream));
-    CK(cudaStreamSynchronize(c->stream));
-    if (m.err & DERR_BAD_GRAPH) return fail(c, CFG_ERR_STATE, "lm-tig ends do not form a valid discontinuity graph");
-    if (m.err & DERR_WALK_LIMIT) return fail(c, CFG_ERR_WALK_LIMIT, "lm-tig ranking exceeded its bound");
     // lm-tigs on closed chains: joined into cycles on the device, rotated to their canonical start
     uint64_t cyc_bytes = 0, cyc_units = 0;
     if (res.n_cycle_lmtigs) {
-        rc = collate_cycles_on_device(c->ub, n.n_lmtig, res.n_cycle_lmtigs, c->p.k, &c->misc.as<MiscWords>()->err,
+        rc = collate_cycles_on_device(c->ub, n.n_lmtig, res.n_cycle_lmtigs, c->p.k, &dev_words(c)->err,
                                       c->cyc_work, c->cyc_scratch, c->cyc_out, c->stream, cyc_bytes, cyc_units);
         if (rc == CFG_ERR_OOM) return fail(c, rc, "cycle buffers");
         if (rc) return fail(c, rc, std::string("cycle collation: ") + cudaGetErrorString(cudaGetLastError()));
-        CK(cudaMemcpyAsync(&m, c->misc.p, sizeof(m), cudaMemcpyDeviceToHost, c->stream));
+        uint32_t err = 0;
+        CK(cudaMemcpyAsync(&err, &dev_words(c)->err, sizeof(err), cudaMemcpyDeviceToHost, c->stream));
         CK(cudaStreamSynchronize(c->stream));
-        if (m.err & DERR_BAD_GRAPH) return fail(c, CFG_ERR_STATE, "lm-tig ends on a closed chain do not pair up");
+        if (err & DERR_BAD_GRAPH) return fail(c, CFG_ERR_STATE, "lm-tig ends on a closed chain do not pair up");
     }
     CK(cudaEventRecord(c->ev[2], c->stream));   // device collation done
     // trivial unitigs (per stripe) + collated unitigs + cycles, to host memory
@@ -777,10 +787,10 @@ void cfg_destroy(cfg_ctx* c) {
     c->parse.release();
     c->ub.release();
     c->h_unitigs.release();
-    DevBuf* bufs[] = {&c->packed, &c->frag_off, &c->frag_len, &c->text, &c->flat, &c->hist, &c->misc, &c->bucket_off, &c->inst, &c->scan_part, &c->rcw,
-                      &c->fill, &c->recs, &c->list, &c->tab_off, &c->tab_cap, &c->arena, &c->fasta, &c->lm_text,
-                      &c->lm, &c->dump, &c->retry, &c->counters, &c->stripe_cur, &c->stripe_base,
-                      &c->ut_lmbase, &c->cyc_work, &c->cyc_scratch, &c->cyc_out};
+    c->h_words.release();
+    DevBuf* bufs[] = {&c->packed, &c->frag_off, &c->frag_len, &c->text, &c->flat, &c->words_d, &c->bucket_off, &c->inst,
+                      &c->scan_part, &c->rcw, &c->recs, &c->list, &c->tab_off, &c->tab_cap, &c->arena, &c->fasta,
+                      &c->lm_text, &c->lm, &c->dump, &c->retry, &c->cyc_work, &c->cyc_scratch, &c->cyc_out};
     for (DevBuf* b : bufs) b->release();
     c->h_fasta.release(); c->h_lm_text.release(); c->h_lm.release();
     for (auto& e : c->ev) if (e) cudaEventDestroy(e);

@@ -28,6 +28,11 @@ constexpr uint32_t SB_MAX_BINS = 1024;    // super-buckets, and subgraphs per su
 constexpr uint32_t SCAN_ITEMS = 8192;     // entries per CTA of the (super-bucket, slab) scan
 constexpr uint32_t UNROLL = 8;            // record loads in flight per thread (a record is never all ones)
 
+// The record count is a device word, so the sort is queued behind the partition without a
+// wait; a count past the buffer (the partition overflowed and is rerun) sorts nothing.
+struct RecCount { const unsigned long long* n; uint64_t cap; };
+__device__ __forceinline__ uint64_t records(const RecCount& c) { const uint64_t n = *c.n; return n > c.cap ? 0 : n; }
+
 __device__ __forceinline__ uint64_t slab_begin(uint64_t n, uint32_t s, uint32_t S) { return n * s / S; }
 
 // Exclusive scan of bins[0..nb) in shared memory (nb <= 1024, blockDim 512); the total
@@ -61,10 +66,11 @@ __device__ void smem_excl_scan(uint32_t* bins, uint32_t nb, uint32_t* warp_sums,
 }
 
 // Pass 1a: counts[h * S + s] = records of slab s in super-bucket h.
-__global__ void __launch_bounds__(SB_THREADS) k_sb_count(const uint64_t* __restrict__ flat, uint64_t n, uint32_t lbits,
+__global__ void __launch_bounds__(SB_THREADS) k_sb_count(const uint64_t* __restrict__ flat, RecCount nr, uint32_t lbits,
                                                          uint32_t H, uint32_t* __restrict__ counts) {
     __shared__ uint32_t cnt[SB_MAX_BINS];
     const uint32_t S = gridDim.x, s = blockIdx.x;
+    const uint64_t n = records(nr);
     for (uint32_t h = threadIdx.x; h < H; h += blockDim.x) cnt[h] = 0;
     __syncthreads();
     const uint64_t e = slab_begin(n, s + 1, S);
@@ -156,7 +162,7 @@ __device__ __forceinline__ void cp_async_wait_all() { asm volatile("cp.async.wai
 // One CTA per SM walks its slab tile by tile with two tile buffers: the copy of tile t+1
 // into one (cp.async) is in flight while tile t is sorted in the other, which then holds
 // the sorted tile until it is written out.
-__global__ void __launch_bounds__(SB_THREADS) k_sb_move_hi(const uint64_t* __restrict__ flat, uint64_t n, uint32_t lbits,
+__global__ void __launch_bounds__(SB_THREADS) k_sb_move_hi(const uint64_t* __restrict__ flat, RecCount nr, uint32_t lbits,
                                                            uint32_t H, const uint32_t* __restrict__ counts,
                                                            uint64_t* __restrict__ tmp) {
     extern __shared__ __align__(16) unsigned char sm[];
@@ -165,6 +171,7 @@ __global__ void __launch_bounds__(SB_THREADS) k_sb_move_hi(const uint64_t* __res
     uint32_t* tcnt = run + SB_MAX_BINS;                               // H: this tile's counts, then offsets
     uint32_t* ws = tcnt + SB_MAX_BINS;                                // scan scratch
     const uint32_t S = gridDim.x, s = blockIdx.x;
+    const uint64_t n = records(nr);
     for (uint32_t h = threadIdx.x; h < H; h += blockDim.x) run[h] = counts[(uint64_t)h * S + s];
     const uint64_t b = slab_begin(n, s, S), e = slab_begin(n, s + 1, S);
     constexpr uint32_t PER = SB_TILE / SB_THREADS;
@@ -218,13 +225,14 @@ __global__ void __launch_bounds__(SB_THREADS) k_sb_move_hi(const uint64_t* __res
 
 // Pass 2: super-bucket h = [base_h, base_{h+1}) of tmp sorted by the low bits of g into
 // out; bucket offsets and k-mer instance counts per subgraph.
-__global__ void __launch_bounds__(SB_THREADS) k_sb_move_lo(const uint64_t* __restrict__ tmp, uint64_t n, uint32_t lbits,
+__global__ void __launch_bounds__(SB_THREADS) k_sb_move_lo(const uint64_t* __restrict__ tmp, RecCount nr, uint32_t lbits,
                                                            uint32_t H, uint32_t S, const uint32_t* __restrict__ counts,
                                                            uint32_t k, uint64_t* __restrict__ out,
                                                            uint32_t* __restrict__ bucket_off, uint32_t* __restrict__ inst) {
     __shared__ uint32_t cnt[SB_MAX_BINS], ins[SB_MAX_BINS], fill[SB_MAX_BINS];
     __shared__ uint32_t ws[SB_THREADS / 32 + 1];
     const uint32_t h = blockIdx.x, L = 1u << lbits, lmask = L - 1;
+    const uint64_t n = records(nr);
     const uint64_t a = counts[(uint64_t)h * S], b = h + 1 < H ? counts[(uint64_t)(h + 1) * S] : n;
     for (uint32_t l = threadIdx.x; l < L; l += blockDim.x) { cnt[l] = 0; ins[l] = 0; fill[l] = 0; }
     __syncthreads();
@@ -274,7 +282,7 @@ uint64_t bucket_sort_scratch_words(uint32_t G, uint32_t sms) {
     return m + (m + SCAN_ITEMS - 1) / SCAN_ITEMS + 1;
 }
 
-cudaError_t launch_bucket_sort(const uint64_t* flat, uint64_t n, uint32_t G, uint32_t k, uint32_t sms, uint32_t* scratch,
+cudaError_t launch_bucket_sort(const uint64_t* flat, const unsigned long long* n_dev, uint64_t cap, uint32_t G, uint32_t k, uint32_t sms, uint32_t* scratch,
                                uint64_t* tmp, uint64_t* out, uint32_t* bucket_off, uint32_t* inst, cudaStream_t s) {
     const uint32_t gbits = 31 - __builtin_clz(G), hbits = gbits < 10 ? gbits : 10, lbits = gbits - hbits;
     const uint32_t H = 1u << hbits, S = sms;   // slabs: one CTA of k_sb_move_hi per SM
@@ -282,6 +290,7 @@ cudaError_t launch_bucket_sort(const uint64_t* flat, uint64_t n, uint32_t G, uin
     uint32_t* counts = scratch;
     uint32_t* sums = scratch + m;
     const uint32_t nsums = (uint32_t)((m + SCAN_ITEMS - 1) / SCAN_ITEMS);
+    const RecCount n{n_dev, cap};
     k_sb_count<<<S, SB_THREADS, 0, s>>>(flat, n, lbits, H, counts);
     k_sb_scan_sums<<<nsums, SB_THREADS, 0, s>>>(counts, m, sums);
     k_sb_scan_apply<<<nsums, SB_THREADS, 0, s>>>(counts, m, sums, nsums);

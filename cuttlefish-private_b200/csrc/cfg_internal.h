@@ -184,9 +184,38 @@ inline uint32_t record_dedup(uint32_t k, uint32_t l, uint32_t cutoff, uint32_t f
 
 constexpr uint32_t OUT_STRIPES = 32;
 
-// Adds each stripe's label-text base to its lm-tigs' label offsets (one job's run).
-void launch_stripe_fixup(LmtigOut* lm, uint64_t lm_slice, const unsigned long long* lm_used,
-                         const unsigned long long* text_base, uint32_t stripes, cudaStream_t s);
+// One job's plan: its subgraphs in launch order, the largest first, made on the device from
+// their k-mer instance counts.  Classes in that order: arena tables, clusters of 8 .. 2 CTAs,
+// one-CTA shapes from the largest; PLAN_SUB size steps within a class.
+constexpr uint32_t PLAN_SHAPES = 12, PLAN_CLASSES = 8 + PLAN_SHAPES, PLAN_SUB = 16, PLAN_BINS = PLAN_CLASSES * PLAN_SUB;
+
+// The small device words of one run, cleared by one memset and read back by one copy.
+struct RunWords {
+    unsigned long long rec_cursor;
+    uint32_t err, pad;
+    uint32_t bins[PLAN_BINS], fill[PLAN_BINS];   // subgraphs per class and size step; placed so far
+    unsigned long long arena_slots, instances;
+    Counters cnt;
+    alignas(128) unsigned long long stripe_cur[JOB_CUR_STRIDE * OUT_STRIPES];
+    unsigned long long lm_base[OUT_STRIPES], text_base[OUT_STRIPES];   // records and label bytes before each stripe
+};
+
+struct PlanArgs {
+    const uint32_t* inst;        // G k-mer instance counts
+    uint32_t G, load, n_shapes, per_cl, max_cluster;
+    int words;
+    uint32_t slots[PLAN_SHAPES];
+    uint32_t* list;              // out: subgraph ids in launch order (those without instances left out)
+    uint64_t* tab_off;           // out, arena tables: slots before the table, and its capacity
+    uint32_t* tab_cap;
+    RunWords* w;                 // out: bins, arena_slots, instances
+};
+void launch_run_plan(const PlanArgs& a, cudaStream_t s);
+
+// After the last pass over a job's subgraphs (no retries, nothing overflowed; otherwise it
+// does nothing): the stripes' bases, and each stripe's label-text base added to its lm-tigs'
+// label offsets.
+void launch_stripe_fixup(LmtigOut* lm, uint64_t lm_slice, RunWords* w, cudaStream_t s);
 
 // Largest k: Kmer<k> of the reference built with INSTANCE_COUNT = 64 (include/globals.hpp:16-22,45).
 constexpr uint32_t MAX_K = 127;
@@ -201,11 +230,11 @@ void launch_partition(const PartitionArgs& a, cudaStream_t s);
 void launch_bucket_scan(const unsigned long long* hist, uint32_t G, uint32_t* bucket_off, uint32_t* inst,
                         uint32_t* fill, cudaStream_t s);
 void launch_scatter(const ScatterArgs& a, cudaStream_t s);
-// Bucket sort of n flat records by subgraph (cfg_bucket_sort.cu) without a global atomic
+// Bucket sort of the *n_dev (at most cap; more: none) flat records by subgraph (cfg_bucket_sort.cu) without a global atomic
 // per record: flat -> tmp (by super-bucket) -> out (by subgraph); bucket_off[0..G] and
 // inst[0..G) come out of it.  scratch: bucket_sort_scratch_words(G, sms) words.
 uint64_t bucket_sort_scratch_words(uint32_t G, uint32_t sms);
-cudaError_t launch_bucket_sort(const uint64_t* flat, uint64_t n, uint32_t G, uint32_t k, uint32_t sms, uint32_t* scratch,
+cudaError_t launch_bucket_sort(const uint64_t* flat, const unsigned long long* n_dev, uint64_t cap, uint32_t G, uint32_t k, uint32_t sms, uint32_t* scratch,
                                uint64_t* tmp, uint64_t* out, uint32_t* bucket_off, uint32_t* inst, cudaStream_t s);
 // cluster == 0: tables in the global arena; 1: one CTA's shared memory; >1: a cluster's.
 cudaError_t launch_subgraphs(const SubgraphArgs& a, int words, uint32_t cluster, uint32_t threads, cudaStream_t s);
@@ -225,7 +254,7 @@ const LocalShape* local_shapes(int words, uint32_t& n);   // one-CTA tables of k
 // vertices).  k <= 31 keeps half load; wider k-mers take two thirds, for the extra CTA or
 // two per SM that the smaller table allows (500 Mbp, k = 63: 132 ms at half load, 110 at
 // 0.57, 98.5 at 0.67, 107 at 0.77; k = 127: 8.7 ms at half load, 7.3 at 0.62).
-inline uint64_t local_fit(int words, uint64_t want) { return words == 1 ? want : want * 3 / 4; }
+__host__ __device__ constexpr uint64_t local_fit(int words, uint64_t want) { return words == 1 ? want : want * 3 / 4; }
 uint32_t subgraph_max_per_cta(int words);      // the largest of them
 // Largest CTA of a launch of `per`-slot tables (per 0: arena tables).
 uint32_t subgraph_max_threads(int words, uint32_t per);

@@ -1470,14 +1470,111 @@ int occupancy_of(K kernel, uint32_t cluster, uint32_t threads, size_t bytes, siz
     return n;
 }
 
-__global__ void k_stripe_fixup(LmtigOut* lm, uint64_t lm_slice, const unsigned long long* __restrict__ lm_used,
-                               const unsigned long long* __restrict__ text_base, uint32_t stripes) {
-    for (uint32_t st = blockIdx.y; st < stripes; st += gridDim.y) {
-        const unsigned long long n = lm_used[st * JOB_CUR_STRIDE + 2];
-        const unsigned long long base = text_base[st];
-        for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n && i < lm_slice; i += (uint64_t)gridDim.x * blockDim.x)
-            lm[st * lm_slice + i].label_off += base;
+__global__ void __launch_bounds__(256) k_stripe_fixup(LmtigOut* lm, uint64_t lm_slice, RunWords* w) {
+    if (w->cnt.retry_count || (w->err & (DERR_OUT_OVERFLOW | DERR_DUMP_OVERFLOW))) return;
+    const uint32_t st = blockIdx.y;
+    unsigned long long base = 0, recs = 0;
+    for (uint32_t q = 0; q < st; ++q) { base += w->stripe_cur[q * JOB_CUR_STRIDE + 1]; recs += w->stripe_cur[q * JOB_CUR_STRIDE + 2]; }
+    if (blockIdx.x == 0 && threadIdx.x == 0) { w->text_base[st] = base; w->lm_base[st] = recs; }
+    const unsigned long long n = w->stripe_cur[st * JOB_CUR_STRIDE + 2];
+    for (uint64_t i = (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; i < n && i < lm_slice; i += (uint64_t)gridDim.x * blockDim.x)
+        lm[st * lm_slice + i].label_off += base;
+}
+
+// ---- the plan of one job's run ----
+// Class (launch order) and size step of a subgraph of n k-mer instances; `want`: the slots
+// it wants, twice its expected vertices.
+__device__ __forceinline__ uint32_t plan_bin(const PlanArgs& a, uint32_t n, uint64_t& want) {
+    want = max(64ull, ((unsigned long long)n * a.load * 2 + 99) / 100);
+    const uint64_t fit = local_fit(a.words, want);
+    uint32_t sh = 0;
+    while (sh < a.n_shapes && a.slots[sh] < fit) ++sh;
+    uint32_t cls, sub;
+    if (sh < a.n_shapes) {
+        const uint32_t hi = a.slots[sh], lo = sh ? a.slots[sh - 1] : 0u;
+        cls = 8 + a.n_shapes - 1 - sh;
+        sub = (uint32_t)((hi - fit) * PLAN_SUB / (hi - lo));
+    } else if (want <= (uint64_t)a.per_cl * a.max_cluster) {
+        const uint32_t cl = (uint32_t)((want + a.per_cl - 1) / a.per_cl);
+        cls = 9 - cl;
+        sub = (uint32_t)(((uint64_t)cl * a.per_cl - want) * PLAN_SUB / a.per_cl);
+    } else {
+        cls = 0;
+        sub = (uint32_t)(max(33, __clzll((long long)want)) - 33);   // a step per doubling, from 2^31 down
     }
+    return cls * PLAN_SUB + min(sub, PLAN_SUB - 1);
+}
+__device__ __forceinline__ uint32_t plan_arena_slots(uint64_t want) {   // the power of two at or above
+    return want > (1ull << 30) ? 1u << 31 : 1u << (64 - __clzll((long long)(want - 1)));
+}
+
+// Subgraphs per bin, instances and arena slots.
+__global__ void __launch_bounds__(256) k_plan_count(const PlanArgs a) {
+    __shared__ uint32_t cnt[PLAN_BINS];
+    for (uint32_t i = threadIdx.x; i < PLAN_BINS; i += blockDim.x) cnt[i] = 0;
+    __syncthreads();
+    const uint32_t g0 = (uint32_t)((uint64_t)a.G * blockIdx.x / gridDim.x), g1 = (uint32_t)((uint64_t)a.G * (blockIdx.x + 1) / gridDim.x);
+    unsigned long long inst = 0;
+    for (uint32_t g = g0 + threadIdx.x; g < g1; g += blockDim.x) {
+        const uint32_t n = a.inst[g];
+        if (!n) continue;
+        inst += n;
+        uint64_t want;
+        atomicAdd(&cnt[plan_bin(a, n, want)], 1u);
+    }
+    for (int d = 16; d; d >>= 1) inst += __shfl_down_sync(0xffffffffu, inst, d);
+    if ((threadIdx.x & 31) == 0 && inst) atomicAdd(&a.w->instances, inst);
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < PLAN_BINS; i += blockDim.x)
+        if (cnt[i]) atomicAdd(&a.w->bins[i], cnt[i]);
+}
+
+// Every subgraph to its place in the launch order (any order within a bin); arena tables
+// are carved out as they come.
+__global__ void __launch_bounds__(256) k_plan_place(const PlanArgs a) {
+    __shared__ uint32_t cnt[PLAN_BINS], at[PLAN_BINS];
+    for (uint32_t i = threadIdx.x; i < PLAN_BINS; i += blockDim.x) cnt[i] = 0;
+    __syncthreads();
+    const uint32_t g0 = (uint32_t)((uint64_t)a.G * blockIdx.x / gridDim.x), g1 = (uint32_t)((uint64_t)a.G * (blockIdx.x + 1) / gridDim.x);
+    uint64_t want;
+    for (uint32_t g = g0 + threadIdx.x; g < g1; g += blockDim.x) {
+        const uint32_t n = a.inst[g];
+        if (n) atomicAdd(&cnt[plan_bin(a, n, want)], 1u);
+    }
+    if (threadIdx.x < 32) {   // bins before each bin
+        constexpr uint32_t PER = PLAN_BINS / 32;
+        uint32_t sum = 0;
+        for (uint32_t j = 0; j < PER; ++j) sum += a.w->bins[threadIdx.x * PER + j];
+        uint32_t x = sum;
+        for (int d = 1; d < 32; d <<= 1) {
+            const uint32_t y = __shfl_up_sync(0xffffffffu, x, d);
+            if (threadIdx.x >= (uint32_t)d) x += y;
+        }
+        x -= sum;
+        for (uint32_t j = 0; j < PER; ++j) { at[threadIdx.x * PER + j] = x; x += a.w->bins[threadIdx.x * PER + j]; }
+    }
+    __syncthreads();
+    for (uint32_t i = threadIdx.x; i < PLAN_BINS; i += blockDim.x)
+        if (cnt[i]) at[i] += atomicAdd(&a.w->fill[i], cnt[i]);
+    __syncthreads();
+    for (uint32_t g = g0 + threadIdx.x; g < g1; g += blockDim.x) {
+        const uint32_t n = a.inst[g];
+        if (!n) continue;
+        const uint32_t b = plan_bin(a, n, want), i = atomicAdd(&at[b], 1u);
+        a.list[i] = g;
+        if (b < PLAN_SUB) {
+            const uint32_t cap = plan_arena_slots(want);
+            a.tab_off[i] = atomicAdd(&a.w->arena_slots, (unsigned long long)cap);
+            a.tab_cap[i] = cap;
+        }
+    }
+}
+static_assert(PLAN_BINS % 32 == 0, "the bin scan gives each lane an equal share");
+
+void launch_run_plan(const PlanArgs& a, cudaStream_t s) {
+    const uint32_t grid = a.G < 512 ? 1u : a.G / 512 < 296 ? a.G / 512 : 296u;
+    k_plan_count<<<grid, 256, 0, s>>>(a);
+    k_plan_place<<<grid, 256, 0, s>>>(a);
 }
 
 const LocalShape* local_shapes(int words, uint32_t& n) {
@@ -1542,9 +1639,8 @@ cudaError_t launch_subgraphs(const SubgraphArgs& a, int words, uint32_t cluster,
     return launch_shared(k_subgraph_shared<1, CLUSTER, 1024>, a, cluster, threads, bytes, s, 0, max_table_bytes<1>());
 }
 
-void launch_stripe_fixup(LmtigOut* lm, uint64_t lm_slice, const unsigned long long* lm_used,
-                         const unsigned long long* text_base, uint32_t stripes, cudaStream_t s) {
-    k_stripe_fixup<<<dim3(64, stripes), 256, 0, s>>>(lm, lm_slice, lm_used, text_base, stripes);
+void launch_stripe_fixup(LmtigOut* lm, uint64_t lm_slice, RunWords* w, cudaStream_t s) {
+    k_stripe_fixup<<<dim3(64, OUT_STRIPES), 256, 0, s>>>(lm, lm_slice, w);
 }
 
 int subgraph_occupancy(int words, uint32_t cluster, uint32_t threads, uint32_t per) {
