@@ -107,7 +107,6 @@ template <> struct KOps<1> {
     __device__ __forceinline__ void push_back(Kmer<1>& x, uint32_t b) const { x.lo = ((x.lo << 2) | b) & mask; }
     __device__ __forceinline__ void push_front(Kmer<1>& x, uint32_t b) const { x.lo = (x.lo >> 2) | ((uint64_t)b << (2 * (k - 1))); }
     __device__ __forceinline__ Kmer<1> rc(const Kmer<1>& x) const { return Kmer<1>{rc_word(x.lo, k)}; }
-    __device__ __forceinline__ uint32_t first_base(const Kmer<1>& x) const { return (uint32_t)(x.lo >> (2 * (k - 1))) & 3; }
     __device__ __forceinline__ uint32_t last_base(const Kmer<1>& x) const { return (uint32_t)x.lo & 3; }
     __device__ __forceinline__ uint32_t base(const Kmer<1>& x, uint32_t i) const { return (uint32_t)(x.lo >> (2 * (k - 1 - i))) & 3; }
     // k bases starting at stream position p
@@ -138,7 +137,6 @@ template <> struct KOps<2> {
         r.lo = (rlo_full << (2 * nh)) | rhi_part;
         return r;
     }
-    __device__ __forceinline__ uint32_t first_base(const Kmer<2>& x) const { return (uint32_t)(x.hi >> (2 * (k - 33))) & 3; }
     __device__ __forceinline__ uint32_t last_base(const Kmer<2>& x) const { return (uint32_t)x.lo & 3; }
     __device__ __forceinline__ uint32_t base(const Kmer<2>& x, uint32_t i) const {
         const uint32_t bp = 2 * (k - 1 - i);
@@ -185,7 +183,6 @@ template <int W> struct KOps {
         o.w[W - 1] = r[W - 1] >> sh;
         return o;
     }
-    __device__ __forceinline__ uint32_t first_base(const Kmer<W>& x) const { return (uint32_t)(x.w[W - 1] >> (2 * (nh - 1))) & 3; }
     __device__ __forceinline__ uint32_t last_base(const Kmer<W>& x) const { return (uint32_t)x.w[0] & 3; }
     __device__ __forceinline__ uint32_t base(const Kmer<W>& x, uint32_t i) const {
         const uint32_t bp = 2 * (k - 1 - i), wi = bp >> 6;
