@@ -230,6 +230,7 @@ struct cfg_batch {
 
     // device collation of all jobs' lm-tigs (cfg_batch_unitigs)
     UnitigBuffers ub;
+    uint64_t ub_lmtigs = 0;             // lm-tigs the collation buffers hold
     DevBuf u_n, u_base, u_out, u_cur, u_err, u_cyc_work, u_cyc_scratch, u_cyc_out;
     std::vector<unsigned long long> h_out_base, h_ucur;
     std::vector<std::string> u_host;    // per job: unitigs joined on the host (cycles; redone jobs)
@@ -816,11 +817,16 @@ int cfg_batch_unitigs(cfg_batch* b, float* device_ms) {
     if (!b->u_n.ensure(8ull * J) || !b->u_base.ensure(8ull * J) || !b->u_out.ensure(8ull * J) ||
         !b->u_cur.ensure(8ull * JOB_CUR_STRIDE * J) || !b->u_err.ensure(16) || !b->ub.ensure_out(out + 16))
         return bfail(b, CFG_ERR_OOM, "collation buffers");
-    // jobs are joined in chunks that fit the free device memory (jobs never join each other)
-    size_t fr = 0, tot = 0;
-    BCK(cudaMemGetInfo(&fr, &tot));
-    const unsigned long long per_lmtig = 240;   // bytes of collation buffers per lm-tig
-    const unsigned long long cap = std::max<unsigned long long>(1ull << 20, (unsigned long long)(fr / 10 * 6) / per_lmtig);
+    // jobs are joined in chunks that fit the free device memory (jobs never join each other);
+    // buffers that already hold every lm-tig need no look at it (cudaMemGetInfo takes 0 to 80 ms
+    // on a host that other processes' GPU calls share)
+    unsigned long long cap = n_all;
+    if (n_all > b->ub_lmtigs) {
+        size_t fr = 0, tot = 0;
+        BCK(cudaMemGetInfo(&fr, &tot));
+        const unsigned long long per_lmtig = 240;   // bytes of collation buffers per lm-tig
+        cap = std::max<unsigned long long>(1ull << 20, (unsigned long long)(fr / 10 * 6) / per_lmtig);
+    }
     BCK(cudaMemcpyAsync(b->u_n.p, jn.data(), 8ull * J, cudaMemcpyHostToDevice, b->stream));
     BCK(cudaMemcpyAsync(b->u_out.p, ob.data(), 8ull * J, cudaMemcpyHostToDevice, b->stream));
     BCK(cudaMemsetAsync(b->u_cur.p, 0, 8ull * JOB_CUR_STRIDE * J, b->stream));
@@ -833,7 +839,8 @@ int cfg_batch_unitigs(cfg_batch* b, float* device_ms) {
         uint32_t j1 = j0;
         unsigned long long n = 0;
         while (j1 < J && (j1 == j0 || n + jn[j1] <= cap)) { jb[j1] = n; n += jn[j1]; ++j1; }
-        if (!b->ub.ensure(n)) return bfail(b, CFG_ERR_OOM, "collation buffers");
+        if (!b->ub.ensure(n)) { b->ub_lmtigs = 0; return bfail(b, CFG_ERR_OOM, "collation buffers"); }
+        b->ub_lmtigs = std::max<uint64_t>(b->ub_lmtigs, n);
         BCK(cudaMemcpyAsync(b->u_base.as<unsigned long long>() + j0, jb.data() + j0, 8ull * (j1 - j0), cudaMemcpyHostToDevice,
                             b->stream));
         BCK(cudaEventRecord(b->ev[0], b->stream));
@@ -884,7 +891,12 @@ int cfg_batch_unitigs(cfg_batch* b, float* device_ms) {
     BCK(cudaStreamSynchronize(b->stream));
     b->unitig_ms = total_ms;
     b->h_out_base.swap(ob);
-    (void)n_all;
+    // the largest job's text fits the page-locked buffer from the first cfg_batch_job_unitigs on
+    uint64_t most = 0;
+    for (uint32_t j = 0; j < J; ++j)
+        if (!b->redo[j])
+            most = std::max<uint64_t>(most, b->h_jobs[j].fasta_used + b->h_ucur[(size_t)j * JOB_CUR_STRIDE] + b->u_host[j].size());
+    (void)b->h_unitigs.ensure(most + 1);   // (where this fails, the job's own call says so)
     // jobs redone alone: their lm-tigs are on the host already
     for (uint32_t j = 0; j < J; ++j) {
         if (!b->redo[j]) continue;
