@@ -362,13 +362,16 @@ struct Block {   // per-CTA shared bookkeeping (in CLUSTER mode the flags of ran
     // overflowed), path ends W1 found, W3's unvisited vertices
     uint32_t fresh_n, w1_n, end_n, cyc_n;
     uint32_t dd_over;   // the record merge's table filled up
+    uint32_t label_n;   // labels left for the whole CTA to write
     unsigned long long vertices, isolated, phantom, trivial, icc, lmtig;
     Sink sk;
     unsigned long long rs[3][32];   // reserve_block: per-warp totals (<= 1024 threads), then their offsets
 };
 
 constexpr uint32_t FULL = 0xffffffffu;
-constexpr uint32_t STEP_BUF = 64;   // bases a path walk keeps for its label (2 bits each)
+// Words of 32 bases (2 bits each) a path walk keeps of its steps for the label: a subgraph's
+// paths rarely hold more than the k - l + 1 k-mers that can share a minimizer.
+template <int W> constexpr int STEP_WORDS = W <= 2 ? 2 : 4;
 
 // Output space reserved for one lane: FASTA bytes, lm-tig records, lm-tig label bytes.
 struct Res { unsigned long long fa, lm_idx, lm_off; };
@@ -666,42 +669,38 @@ struct RecWords {
     }
 };
 
-// A path of n vertices from v0 (leaving through side0) to vlast, written into space
-// reserved by reserve_warp: a trivial maximal unitig at FASTA offset fo, or an lm-tig
-// (lm: one end exits the subgraph) as record idx with its label at offset off.
-// The label of a path whose bases the walk kept: the walk's first k-mer, then one base
-// per step; `skip` leading bases are not part of the path (a one-k-mer cycle at its start).
-
-// The walk's bases as a little-endian 2-bit array over four words: base j at bits
-// 2 (j & 31) of word j >> 5 (first k-mer, then up to 64 steps: at most 127 bases).
-struct WalkSeq { uint64_t w0, w1, w2, w3; };
+// The label of a path whose bases the walk kept: its first k-mer, then one base per step, as
+// a little-endian 2-bit array (base j at bits 2 (j & 31) of word j >> 5).  `skip` leading
+// bases are not part of the path (a one-k-mer cycle at its start); the L after them go to dst,
+// or (rev) their reverse complement.  Kept in shared memory until the whole CTA writes it.
+template <int W> struct Label {
+    static constexpr int NQ = W + STEP_WORDS<W>;
+    uint64_t q[NQ];
+    unsigned long long dst;
+    uint32_t L, skip_rev;   // skip << 1 | rev
+};
 __device__ __forceinline__ uint64_t rev_bases(uint64_t x) {   // reverses the order of 32 2-bit bases
     const uint64_t r = __brevll(x);
     return ((r >> 1) & 0x5555555555555555ull) | ((r & 0x5555555555555555ull) << 1);
 }
 template <int W>
-__device__ __forceinline__ WalkSeq walk_seq(uint32_t k, const Kmer<W>& first, uint64_t s0, uint64_t s1) {
-    WalkSeq q;
-    if constexpr (W == 1) {   // k <= 31
-        const uint32_t sh = 2 * k;
-        const uint64_t f = rev_bases(first.lo) >> (64 - sh);
-        q.w0 = f | (s0 << sh); q.w1 = (s0 >> (64 - sh)) | (s1 << sh); q.w2 = s1 >> (64 - sh); q.w3 = 0;
-    } else if constexpr (W == 2) {   // 33 <= k <= 63: hi holds the first k - 32 bases
-        const uint32_t sh = 2 * (k - 32);
-        const uint64_t h = rev_bases(first.hi) >> (64 - sh), lo = rev_bases(first.lo);
-        q.w0 = h | (lo << sh); q.w1 = (lo >> (64 - sh)) | (s0 << sh);
-        q.w2 = (s0 >> (64 - sh)) | (s1 << sh); q.w3 = s1 >> (64 - sh);
-    } else {                  // k > 63 keeps no buffered labels (first k-mer + steps exceed 128 bases)
-        q.w0 = q.w1 = q.w2 = q.w3 = 0;
+__device__ __forceinline__ void label_bases(uint64_t (&q)[Label<W>::NQ], uint32_t k, const Kmer<W>& first,
+                                            const uint64_t (&steps)[STEP_WORDS<W>]) {
+    const uint32_t sh = 2 * (k - 32 * (W - 1));   // 2..62 bits: the bases of the highest word
+    uint64_t cur = rev_bases(first.word(W - 1)) >> (64 - sh);
+#pragma unroll
+    for (int i = 0; i < W + STEP_WORDS<W>; ++i) {
+        const uint64_t next = i < W - 1 ? rev_bases(first.word(i < W - 1 ? W - 2 - i : 0))
+                            : i < W - 1 + STEP_WORDS<W> ? steps[i >= W - 1 && i < W - 1 + STEP_WORDS<W> ? i - (W - 1) : 0] : 0ull;
+        q[i] = cur | (next << sh);
+        cur = next >> (64 - sh);
     }
-    return q;
 }
-// bases j .. j+7 (j + 8 <= 128), base j in bits 1:0
-__device__ __forceinline__ uint32_t seq_get16(const WalkSeq& q, uint32_t j) {
+// bases j .. j+7 of a label, base j in bits 1:0
+template <int N> __device__ __forceinline__ uint32_t label_get8(const uint64_t (&q)[N], uint32_t j) {
     const uint32_t w = j >> 5, o = 2 * (j & 31);
-    const uint64_t a = w == 0 ? q.w0 : w == 1 ? q.w1 : w == 2 ? q.w2 : q.w3;
-    const uint64_t b = w == 0 ? q.w1 : w == 1 ? q.w2 : w == 2 ? q.w3 : 0ull;
-    const uint64_t v = o ? ((a >> o) | (b << (64 - o))) : a;
+    uint64_t v = q[w] >> o;
+    if (o > 48) v |= q[w + 1 < N ? w + 1 : w] << (64 - o);
     return (uint32_t)v & 0xFFFFu;
 }
 // character tables for __byte_perm: byte b is the character of base b (or of its complement)
@@ -717,46 +716,47 @@ __device__ __forceinline__ uint32_t rev8bases(uint32_t x16) {   // reverses the 
     const uint32_t r = __brev(x16) >> 16;
     return ((r >> 1) & 0x5555u) | ((r & 0x5555u) << 1);
 }
-
-// Output byte i is base skip + i (forward), or the complement of base skip + L - 1 - i
-// (rev); written in address order, eight characters per aligned 8-byte store.
-template <int W>
-__device__ void write_buffered(const KOps<W>& ops, const Kmer<W>& first, unsigned long long steps0,
-                               unsigned long long steps1, uint32_t skip, uint32_t L, char* dst, bool rev) {
-    if (!dst || W > 2) return;
-    const WalkSeq q = walk_seq<W>(ops.k, first, steps0, steps1);
+// A label written by LABEL_LANES<W> neighbouring threads, 8 aligned bytes at a time in turn.
+// Left to the thread that walked it, a label is 5 to 30 words one after another in the few
+// warps that hold path ends, while the CTA's other warps wait; spread over the CTA: 12 Mbp
+// k = 127 (labels of 180 bases, before re-walked past 64 vertices) subgraphs 5.86 -> 3.92 ms,
+// 500 Mbp k = 63 68.9 -> 66.4, 5 Mbp k = 31 0.70 -> 0.66, reads30x 27.1 -> 26.9.  Lanes per label,
+// k = 31 (36 to 60 bases): 32 cost more than they save (24 Mbp 2.79 -> 3.43 ms), 8 2.86, 2 2.80.
+template <int W> constexpr uint32_t LABEL_LANES = W == 1 ? 2 : W == 2 ? 8 : 32;
+template <int W> __device__ __forceinline__ void write_label(const Label<W>& b, uint32_t lane) {
+    const uint32_t L = b.L, skip = b.skip_rev >> 1, off = (uint32_t)(b.dst & 7);
+    const bool rev = b.skip_rev & 1;
     const uint32_t table = rev ? CH_CMP : CH_FWD;
-    auto one = [&](uint32_t i) {
-        const uint32_t b = seq_get16(q, rev ? skip + L - 1 - i : skip + i) & 3u;
-        dst[i] = (char)(table >> (8 * b));
-    };
-    const uint32_t off = (uint32_t)((unsigned long long)dst & 7);
-    const uint32_t head = off ? (L < 8 - off ? L : 8 - off) : 0;
-    uint32_t i = 0;
-    for (; i < head; ++i) one(i);
-    for (; i + 8 <= L; i += 8) {
-        const uint32_t x = rev ? rev8bases(seq_get16(q, skip + L - 8 - i)) : seq_get16(q, skip + i);
-        *(unsigned long long*)(dst + i) = chars8(x, table);
+    for (uint32_t c = lane; 8 * c < L + off; c += LABEL_LANES<W>) {
+        char* p = (char*)(b.dst - off) + 8 * c;
+        const int32_t i0 = (int32_t)(8 * c) - (int32_t)off;   // the label byte at p
+        if (i0 >= 0 && i0 + 8 <= (int32_t)L) {
+            const uint32_t x = rev ? rev8bases(label_get8(b.q, skip + L - 8 - i0)) : label_get8(b.q, skip + i0);
+            *(unsigned long long*)p = chars8(x, table);
+        } else {
+            const int32_t lo = i0 < 0 ? -i0 : 0, hi = i0 + 8 <= (int32_t)L ? 8 : (int32_t)L - i0;
+            for (int32_t j = lo; j < hi; ++j) {
+                const uint32_t at = rev ? skip + L - 1 - (i0 + j) : skip + i0 + j;
+                p[j] = (char)(table >> (8 * ((b.q[at >> 5] >> (2 * (at & 31))) & 3)));
+            }
+        }
     }
-    for (; i < L; ++i) one(i);
 }
 
+// A path of n vertices from v0 (leaving through side0) to vlast in the space reserved for it: a
+// trivial maximal unitig at FASTA offset fo, or an lm-tig (lm: one end exits the subgraph) as
+// record idx with its label at offset off.  Writes all but the label; where that goes, and in
+// which strand, is returned (dst 0: no room).
+struct LabelOut { char* dst; bool rev; };
 template <int W, int MODE>
-__device__ void write_emitted_path(const SubgraphArgs& a, const Tab<W, MODE>& T, const KOps<W>& ops, const DV<W>& v0,
-                                   int side0, uint32_t n, const DV<W>& vlast, EndInfo st, EndInfo en, bool seed_canon,
-                                   Block& B, bool lm, unsigned long long fo, unsigned long long idx,
-                                   unsigned long long off, bool buffered, unsigned long long steps0,
-                                   unsigned long long steps1, const Kmer<W>& first, uint32_t skip, bool links) {
-    const uint32_t k = ops.k, fth = a.fth;
-    const uint32_t L = n + k - 1;
+__device__ LabelOut emit_path(const Tab<W, MODE>& T, const KOps<W>& ops, const DV<W>& v0, uint32_t n, const DV<W>& vlast,
+                              EndInfo st, EndInfo en, bool seed_canon, Block& B, bool lm, unsigned long long fo,
+                              unsigned long long idx, unsigned long long off) {
+    const uint32_t L = n + ops.k - 1;
     if (!lm) {
         // trivial maximal unitig in canonical orientation (Maximal_Unitig_Scratch::finalize, :200-222)
-        const bool rev = vlast.r < v0.d;   // rc(last k-mer) < first k-mer
-        char* p = fasta_at(B.sk, fo, L);
-        if (buffered) write_buffered(ops, first, steps0, steps1, skip, L, p, rev);
-        else write_path(T, ops, fth, v0, side0, n, p, rev, true, links);
         atomicAdd(&B.trivial, 1ull);
-        return;
+        return LabelOut{fasta_at(B.sk, fo, L), vlast.r < v0.d};   // rc(last k-mer) < first k-mer
     }
     // lm-tig oriented by its first-inserted vertex (finalize_weak, :225-233; Unitig_File add, include/Unitig_File.hpp:338-359)
     const bool rev = !seed_canon;
@@ -765,11 +765,7 @@ __device__ void write_emitted_path(const SubgraphArgs& a, const Tab<W, MODE>& T,
     const bool v_last_canon = rev ? !st.canon : en.canon;      // label's last k-mer canonical?
     const Sink& sk = B.sk;
     atomicAdd(&B.lmtig, 1ull);
-    const bool fits = idx < sk.lm_cap && off + L <= sk.lm_text_cap;
-    if (!fits) atomicOr(sk.oflow, DERR_OUT_OVERFLOW);
-    if (buffered) write_buffered(ops, first, steps0, steps1, skip, L, fits ? sk.lm_text + off : nullptr, rev);
-    else write_path(T, ops, fth, v0, side0, n, fits ? sk.lm_text + off : nullptr, rev, true, links);
-    if (!fits) return;
+    if (!(idx < sk.lm_cap && off + L <= sk.lm_text_cap)) { atomicOr(sk.oflow, DERR_OUT_OVERFLOW); return LabelOut{nullptr, rev}; }
     LmtigOut o;
     const Kmer<W> phi = phi_kmer(ops);
     const bool u_exit = eu.term == T_EXIT, v_exit = ev.term == T_EXIT;
@@ -781,6 +777,7 @@ __device__ void write_emitted_path(const SubgraphArgs& a, const Tab<W, MODE>& T,
     o.flags = (uint8_t)(s_u_back | (s_v_back << 1) | ((!u_exit) << 2) | ((!v_exit) << 3));
     o.pad = 0;
     sk.lm[idx] = o;
+    return LabelOut{sk.lm_text + off, rev};
 }
 
 // rank/nranks: this CTA's position in its cluster; per: slots owned by one CTA.
@@ -1121,13 +1118,17 @@ __device__ void run_subgraph(const SubgraphArgs& a, const Tab<W, MODE>& T, Block
         __syncthreads();
     }
     const uint32_t nw2 = ends_listed ? n_ends : *(volatile uint32_t*)&B.end_n;
+    // labels wait in what W1's list has left free of wl
+    const uint32_t free0 = ends_top ? 0u : nw2, free1 = ends_top ? per - n_ends : per;
+    Label<W>* const labels = (Label<W>*)(((unsigned long long)(wl + free0) + 7) & ~7ull);
+    const uint32_t label_cap = (free1 - free0) * 4 < sizeof(Label<W>) + 8 ? 0u : ((free1 - free0) * 4 - 8) / (uint32_t)sizeof(Label<W>);
     uint32_t n_cov = 0;   // vertices of what this thread emitted
     for (uint32_t base = 0; base < nw2; base += nt) {   // uniform over the CTA: warps reserve output together
         const uint32_t i = base + tid;
         // what this lane emits: one-k-mer cycles at s and/or e, and one path vs..ve
         bool kc0 = false, kc1 = false, mark0 = false, mark1 = false, path = false, lm = false;
         uint32_t s = 0, e = 0, n2 = 0, walked = 0;   // walked: vertices of the two-end walk (0: one vertex)
-        unsigned long long steps0 = 0, steps1 = 0;   // bases of walk steps 1..32, 33..64
+        uint64_t steps[STEP_WORDS<W>] = {};          // bases of walk steps 1..32, 33..64, ...
         Kmer<W> first{};
         DV<W> vs{}, ve{};
         int sd0 = BACK;
@@ -1151,8 +1152,8 @@ __device__ void run_subgraph(const SubgraphArgs& a, const Tab<W, MODE>& T, Block
                 const uint32_t ins0 = st_ins(lst[sti<W>(ls)]);
                 const DV<W> v0 = dv_at(T, ops, s, side0);
                 // pass 1: the other end, first-occurrence minima; the walk marks its vertices
-                // and keeps the bases it steps through (2 bits each, up to STEP_BUF of them),
-                // so the emitting end writes its label without walking again
+                // and keeps the bases it steps through (2 bits each, up to STEP_WORDS words of
+                // them), so the label is written without walking again
                 DV<W> v = v0; int side = side0;
                 uint32_t n = 1;
                 uint32_t v1_slot = s; int v1_side = side0;     // second vertex
@@ -1183,9 +1184,11 @@ __device__ void run_subgraph(const SubgraphArgs& a, const Tab<W, MODE>& T, Block
                     side = 1 - s_in;
                     cur_meta = T.ld_meta(v.slot);
                     T.or_meta(v.slot, M_VISITED);
-                    if (n <= STEP_BUF) {
-                        const unsigned long long bb = (unsigned long long)b << (2 * ((n - 1) & 31));
-                        if (n <= 32) steps0 |= bb; else steps1 |= bb;
+                    {
+                        const uint64_t bb = (uint64_t)b << (2 * ((n - 1) & 31));
+#pragma unroll
+                        for (uint32_t j = 0; j < STEP_WORDS<W>; ++j)
+                            if ((n - 1) >> 5 == j) steps[j] |= bb;
                     }
                     if (n == 1) { v1_slot = v.slot; v1_side = side; }
                     if (++n > T.per * T.nranks + 1) { atomicOr(a.err, DERR_WALK_LIMIT); ok = false; break; }
@@ -1222,6 +1225,7 @@ __device__ void run_subgraph(const SubgraphArgs& a, const Tab<W, MODE>& T, Block
             if (path) lm = st.term == T_EXIT || en.term == T_EXIT;
         }
         const uint32_t L = path ? n2 + k - 1 : 0;
+        if (tid == 0) B.label_n = 0;
         __syncwarp();
         const Res r = reserve_block(B.sk, B, (kc0 ? k + 4 : 0) + (kc1 ? k + 4 : 0) + (path && !lm ? L + 4 : 0),
                                    path && lm ? 1u : 0u, path && lm ? L : 0u);
@@ -1229,10 +1233,20 @@ __device__ void run_subgraph(const SubgraphArgs& a, const Tab<W, MODE>& T, Block
         if (kc0) { write_kmer_cycle(T, ops, s, B, fo); fo += k + 4; }
         if (kc1) { write_kmer_cycle(T, ops, e, B, fo); fo += k + 4; }
         if (path) {
-            const bool buffered = W <= 2 && walked > 0 && walked - 1 <= STEP_BUF;
-            write_emitted_path(a, T, ops, vs, sd0, n2, ve, st, en, best_canon, B, lm, fo, r.lm_idx, r.lm_off,
-                               buffered, steps0, steps1, first, kc0 ? 1u : 0u, links);
+            const LabelOut o = emit_path(T, ops, vs, n2, ve, st, en, best_canon, B, lm, fo, r.lm_idx, r.lm_off);
+            const bool kept = walked > 0 && walked - 1 <= 32 * STEP_WORDS<W>;   // the walk marked the path and has its bases
+            const uint32_t at = kept && o.dst ? atomicAdd(&B.label_n, 1u) : 0u;
+            if (!kept || (o.dst && at >= label_cap)) write_path(T, ops, fth, vs, sd0, n2, o.dst, o.rev, true, links);
+            else if (o.dst) {
+                Label<W>& b = labels[at];
+                label_bases<W>(b.q, k, first, steps);
+                b.dst = (unsigned long long)o.dst; b.L = L; b.skip_rev = (kc0 ? 2u : 0u) | (o.rev ? 1u : 0u);
+            }
         }
+        __syncthreads();
+        const uint32_t n_labels = min(*(volatile uint32_t*)&B.label_n, label_cap);
+        for (uint32_t j = tid / LABEL_LANES<W>; j < n_labels; j += nt / LABEL_LANES<W>) write_label<W>(labels[j], tid % LABEL_LANES<W>);
+        __syncthreads();   // labels, and their count, are read before the next turn
         if (mark0) T.or_meta(s, M_VISITED);
         if (mark1) T.or_meta(e, M_VISITED);
         n_cov += (kc0 ? 1u : 0u) + (kc1 ? 1u : 0u) + (path ? n2 : 0u);
