@@ -186,9 +186,9 @@ template <int W> struct KOps {
     __device__ __forceinline__ uint32_t last_base(const Kmer<W>& x) const { return (uint32_t)x.w[0] & 3; }
     __device__ __forceinline__ uint32_t base(const Kmer<W>& x, uint32_t i) const {
         const uint32_t bp = 2 * (k - 1 - i), wi = bp >> 6;
-        uint64_t v = x.w[0];
+        uint64_t v = 0;
 #pragma unroll
-        for (int j = 1; j < W; ++j) v = wi == (uint32_t)j ? x.w[j] : v;   // a select, not an indexed load
+        for (int j = 0; j < W; ++j) v |= wi == (uint32_t)j ? x.w[j] : 0ull;   // selects, not an indexed load
         return (uint32_t)(v >> (bp & 63)) & 3;
     }
     __device__ __forceinline__ Kmer<W> load(const uint64_t* s, uint64_t p) const {

@@ -634,9 +634,9 @@ struct RecWords {
         return r;
     }
     __device__ __forceinline__ uint64_t word(uint32_t i) const {   // word i, 0 past the end
-        uint64_t v = 0;
+        uint64_t v = 0;   // an OR of selects: a chain of them would become an array in local memory
 #pragma unroll
-        for (int x = 0; x < NW; ++x) v = i == (uint32_t)x ? w[x] : v;
+        for (int x = 0; x < NW; ++x) v |= i == (uint32_t)x ? w[x] : 0ull;
         return v;
     }
     __device__ __forceinline__ uint64_t bases64(uint32_t i) const {   // bases i .. i+31, base i at 63:62
@@ -716,18 +716,12 @@ __device__ __forceinline__ uint32_t rev8bases(uint32_t x16) {   // reverses the 
     const uint32_t r = __brev(x16) >> 16;
     return ((r >> 1) & 0x5555u) | ((r & 0x5555u) << 1);
 }
-// A label written by LABEL_LANES<W> neighbouring threads, 8 aligned bytes at a time in turn.
-// Left to the thread that walked it, a label is 5 to 30 words one after another in the few
-// warps that hold path ends, while the CTA's other warps wait; spread over the CTA: 12 Mbp
-// k = 127 (labels of 180 bases, before re-walked past 64 vertices) subgraphs 5.86 -> 3.92 ms,
-// 500 Mbp k = 63 68.9 -> 66.4, 5 Mbp k = 31 0.70 -> 0.66, reads30x 27.1 -> 26.9.  Lanes per label,
-// k = 31 (36 to 60 bases): 32 cost more than they save (24 Mbp 2.79 -> 3.43 ms), 8 2.86, 2 2.80.
-template <int W> constexpr uint32_t LABEL_LANES = W == 1 ? 2 : W == 2 ? 8 : 32;
-template <int W> __device__ __forceinline__ void write_label(const Label<W>& b, uint32_t lane) {
+// A label written by LANES neighbouring threads, 8 aligned bytes at a time in turn.
+template <int W, uint32_t LANES> __device__ __forceinline__ void write_label(const Label<W>& b, uint32_t lane) {
     const uint32_t L = b.L, skip = b.skip_rev >> 1, off = (uint32_t)(b.dst & 7);
     const bool rev = b.skip_rev & 1;
     const uint32_t table = rev ? CH_CMP : CH_FWD;
-    for (uint32_t c = lane; 8 * c < L + off; c += LABEL_LANES<W>) {
+    for (uint32_t c = lane; 8 * c < L + off; c += LANES) {
         char* p = (char*)(b.dst - off) + 8 * c;
         const int32_t i0 = (int32_t)(8 * c) - (int32_t)off;   // the label byte at p
         if (i0 >= 0 && i0 + 8 <= (int32_t)L) {
@@ -1186,9 +1180,8 @@ __device__ void run_subgraph(const SubgraphArgs& a, const Tab<W, MODE>& T, Block
                     T.or_meta(v.slot, M_VISITED);
                     {
                         const uint64_t bb = (uint64_t)b << (2 * ((n - 1) & 31));
-#pragma unroll
-                        for (uint32_t j = 0; j < STEP_WORDS<W>; ++j)
-                            if ((n - 1) >> 5 == j) steps[j] |= bb;
+#pragma unroll   // (selects: a conditional |= would put the words in local memory)
+                        for (uint32_t j = 0; j < STEP_WORDS<W>; ++j) steps[j] |= (n - 1) >> 5 == j ? bb : 0ull;
                     }
                     if (n == 1) { v1_slot = v.slot; v1_side = side; }
                     if (++n > T.per * T.nranks + 1) { atomicOr(a.err, DERR_WALK_LIMIT); ok = false; break; }
@@ -1235,18 +1228,31 @@ __device__ void run_subgraph(const SubgraphArgs& a, const Tab<W, MODE>& T, Block
         if (path) {
             const LabelOut o = emit_path(T, ops, vs, n2, ve, st, en, best_canon, B, lm, fo, r.lm_idx, r.lm_off);
             const bool kept = walked > 0 && walked - 1 <= 32 * STEP_WORDS<W>;   // the walk marked the path and has its bases
-            const uint32_t at = kept && o.dst ? atomicAdd(&B.label_n, 1u) : 0u;
-            if (!kept || (o.dst && at >= label_cap)) write_path(T, ops, fth, vs, sd0, n2, o.dst, o.rev, true, links);
-            else if (o.dst) {
-                Label<W>& b = labels[at];
+            auto fill = [&](Label<W>& b) {
                 label_bases<W>(b.q, k, first, steps);
                 b.dst = (unsigned long long)o.dst; b.L = L; b.skip_rev = (kc0 ? 2u : 0u) | (o.rev ? 1u : 0u);
+            };
+            if (!kept) write_path(T, ops, fth, vs, sd0, n2, o.dst, o.rev, true, links);
+            else if (o.dst) {
+                const uint32_t at = MODE == CLUSTER ? NONE : atomicAdd(&B.label_n, 1u);
+                if (at < label_cap) fill(labels[at]);
+                else { Label<W> own; fill(own); write_label<W, 1>(own, 0); }
             }
         }
-        __syncthreads();
-        const uint32_t n_labels = min(*(volatile uint32_t*)&B.label_n, label_cap);
-        for (uint32_t j = tid / LABEL_LANES<W>; j < n_labels; j += nt / LABEL_LANES<W>) write_label<W>(labels[j], tid % LABEL_LANES<W>);
-        __syncthreads();   // labels, and their count, are read before the next turn
+        // Left to the thread that walked it, a label is 5 to 30 words one after another in the
+        // few warps that hold path ends, while the CTA's other warps wait; by the whole CTA:
+        // 12 Mbp k = 127 (labels of 180 bases, before re-walked past 64 vertices) subgraphs 5.82 ->
+        // 3.68 ms, 500 Mbp k = 63 67.2 -> 66.0, 5 Mbp k = 31 0.70 -> 0.65, reads30x 27.1 -> 26.8.
+        // Lanes per label at k = 31 (36 to 60 bases): with 32 they cost more than they save (24 Mbp
+        // 2.79 -> 3.43 ms), 8 2.86, 2 2.79.  A cluster's emitting ends crowd its first CTA, whose
+        // threads each have a label of their own, and write it.
+        if constexpr (MODE != CLUSTER) {
+            __syncthreads();
+            constexpr uint32_t LANES = W == 1 ? 2 : W == 2 ? 8 : 32;
+            const uint32_t n_labels = min(*(volatile uint32_t*)&B.label_n, label_cap);
+            for (uint32_t j = tid / LANES; j < n_labels; j += nt / LANES) write_label<W, LANES>(labels[j], tid % LANES);
+            __syncthreads();   // labels, and their count, are read before the next turn
+        }
         if (mark0) T.or_meta(s, M_VISITED);
         if (mark1) T.or_meta(e, M_VISITED);
         n_cov += (kc0 ? 1u : 0u) + (kc1 ? 1u : 0u) + (path ? n2 : 0u);
