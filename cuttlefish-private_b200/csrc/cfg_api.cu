@@ -277,7 +277,7 @@ int launch_retries(cfg_ctx* c, const std::vector<uint32_t>& work, const std::vec
     std::vector<uint32_t> cap;
     uint64_t arena_slots = 0;
     for (size_t i = 0; i < work.size(); ++i) {
-        const uint64_t w = want[i], fit = local_fit(c->words, w);
+        const uint64_t w = want[i], fit = local_fit(c->words, pa.load, w);
         uint32_t sh = 0;
         while (sh < n_shapes && shapes[sh].slots < fit) ++sh;
         if (sh < n_shapes) of[9 + sh].push_back(work[i]);

@@ -250,11 +250,18 @@ void launch_bucket_scan_large(const unsigned long long* hist, uint32_t n, uint32
                               uint32_t* fill, uint32_t* partials, cudaStream_t s);
 struct LocalShape { uint32_t slots, threads; };
 const LocalShape* local_shapes(int words, uint32_t& n);   // one-CTA tables of k-mers of `words` words, smallest first
-// Slots a one-CTA table must have for a subgraph that wants `want` (twice its expected
-// vertices).  k <= 31 keeps half load; wider k-mers take two thirds, for the extra CTA or
-// two per SM that the smaller table allows (500 Mbp, k = 63: 132 ms at half load, 110 at
-// 0.57, 98.5 at 0.67, 107 at 0.77; k = 127: 8.7 ms at half load, 7.3 at 0.62).
-__host__ __device__ constexpr uint64_t local_fit(int words, uint64_t want) { return words == 1 ? want : want * 3 / 4; }
+// Slots a one-CTA table must have for a subgraph that wants `want` (twice the vertices that
+// `load` percent of its instances make).  A load of 100 or more is a bound, not a guess, and
+// a fuller table lets more CTAs share an SM: k > 32 tables fill to two thirds (500 Mbp, k = 63:
+// 132 ms half full, 110 at 0.57, 98.5 at 0.67, 107 at 0.77; k = 127: 8.7 half full, 7.3 at
+// 0.62); k <= 31 to 0.62 past 4096 slots, where half full means one CTA per SM or a cluster
+// (24 Mbp, k = 23: 2.78 -> 2.72 ms, 60 Mbp on 16384 subgraphs 13.8 -> 10.2), and to half below
+// (8 Mbp, 570 instances a subgraph: 0.92 ms, 1.06 at 0.62).  Under 100 (read sets) the guess
+// may be low, and a table that overflows is built twice: half (reads at k = 47: 4.3 ms, 5.0
+// at two thirds).
+__host__ __device__ constexpr uint64_t local_fit(int words, uint32_t load, uint64_t want) {
+    return load < 100 ? want : words > 1 ? want * 3 / 4 : want > 4096 ? want * 13 / 16 : want;
+}
 uint32_t subgraph_max_per_cta(int words);      // the largest of them
 // Largest CTA of a launch of `per`-slot tables (per 0: arena tables).
 uint32_t subgraph_max_threads(int words, uint32_t per);

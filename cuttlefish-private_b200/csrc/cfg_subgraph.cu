@@ -1490,7 +1490,7 @@ __global__ void __launch_bounds__(256) k_stripe_fixup(LmtigOut* lm, uint64_t lm_
 // it wants, twice its expected vertices.
 __device__ __forceinline__ uint32_t plan_bin(const PlanArgs& a, uint32_t n, uint64_t& want) {
     want = max(64ull, ((unsigned long long)n * a.load * 2 + 99) / 100);
-    const uint64_t fit = local_fit(a.words, want);
+    const uint64_t fit = local_fit(a.words, a.load, want);
     uint32_t sh = 0;
     while (sh < a.n_shapes && a.slots[sh] < fit) ++sh;
     uint32_t cls, sub;
