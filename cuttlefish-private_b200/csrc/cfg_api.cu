@@ -190,7 +190,7 @@ int run_partition(cfg_ctx* c) {
         CK(cudaEventRecord(c->ev[3], c->stream));
         // flat -> recs (by super-bucket) -> flat (by subgraph), then the two buffers trade
         // places: c->recs holds the bucketed records, c->flat the next run's partition output
-        CK(launch_bucket_sort(c->flat.as<uint64_t>(), a.rec_cursor, cap, G, c->p.k, c->sms, c->scan_part.as<uint32_t>(),
+        CK(launch_bucket_sort(c->flat.as<uint64_t>(), a.rec_cursor, cap, c->n_bases, G, c->p.k, c->sms, c->scan_part.as<uint32_t>(),
                               c->recs.as<uint64_t>(), c->flat.as<uint64_t>(), c->bucket_off.as<uint32_t>(),
                               c->inst.as<uint32_t>(), c->stream));
         CK(cudaEventRecord(c->ev[4], c->stream));

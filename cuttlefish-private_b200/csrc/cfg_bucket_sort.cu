@@ -112,10 +112,11 @@ __global__ void __launch_bounds__(SB_THREADS) k_sb_scan_apply(uint32_t* __restri
                                                               const uint32_t* __restrict__ sums, uint32_t nsums) {
     __shared__ uint32_t items[SCAN_ITEMS];
     __shared__ uint32_t ws[SB_THREADS / 32], base;
-    if (threadIdx.x == 0) {
+    if (threadIdx.x < 32) {   // the blocks before this one
         uint32_t b = 0;
-        for (uint32_t i = 0; i < blockIdx.x && i < nsums; ++i) b += sums[i];
-        base = b;
+        for (uint32_t i = threadIdx.x; i < blockIdx.x && i < nsums; i += 32) b += sums[i];
+        b = __reduce_add_sync(0xffffffffu, b);
+        if (threadIdx.x == 0) base = b;
     }
     const uint64_t b0 = (uint64_t)blockIdx.x * SCAN_ITEMS;
     for (uint32_t i = threadIdx.x; i < SCAN_ITEMS; i += blockDim.x) items[i] = b0 + i < m ? v[b0 + i] : 0u;
@@ -282,10 +283,13 @@ uint64_t bucket_sort_scratch_words(uint32_t G, uint32_t sms) {
     return m + (m + SCAN_ITEMS - 1) / SCAN_ITEMS + 1;
 }
 
-cudaError_t launch_bucket_sort(const uint64_t* flat, const unsigned long long* n_dev, uint64_t cap, uint32_t G, uint32_t k, uint32_t sms, uint32_t* scratch,
+cudaError_t launch_bucket_sort(const uint64_t* flat, const unsigned long long* n_dev, uint64_t cap, uint64_t n_bases, uint32_t G, uint32_t k, uint32_t sms, uint32_t* scratch,
                                uint64_t* tmp, uint64_t* out, uint32_t* bucket_off, uint32_t* inst, cudaStream_t s) {
     const uint32_t gbits = 31 - __builtin_clz(G), hbits = gbits < 10 ? gbits : 10, lbits = gbits - hbits;
-    const uint32_t H = 1u << hbits, S = sms;   // slabs: one CTA of k_sb_move_hi per SM
+    // slabs: one CTA of k_sb_move_hi per SM, but some 2048 records each at least (6 bases a
+    // record): the (super-bucket, slab) counts of a 50 kbp job are then 5 k, not 151 k, to scan
+    const uint64_t slabs = n_bases / (6 * 2048) + 1;
+    const uint32_t H = 1u << hbits, S = (uint32_t)(slabs < sms ? slabs : sms);
     const uint64_t m = (uint64_t)H * S;
     uint32_t* counts = scratch;
     uint32_t* sums = scratch + m;

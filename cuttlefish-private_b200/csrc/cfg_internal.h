@@ -234,7 +234,7 @@ void launch_scatter(const ScatterArgs& a, cudaStream_t s);
 // per record: flat -> tmp (by super-bucket) -> out (by subgraph); bucket_off[0..G] and
 // inst[0..G) come out of it.  scratch: bucket_sort_scratch_words(G, sms) words.
 uint64_t bucket_sort_scratch_words(uint32_t G, uint32_t sms);
-cudaError_t launch_bucket_sort(const uint64_t* flat, const unsigned long long* n_dev, uint64_t cap, uint32_t G, uint32_t k, uint32_t sms, uint32_t* scratch,
+cudaError_t launch_bucket_sort(const uint64_t* flat, const unsigned long long* n_dev, uint64_t cap, uint64_t n_bases, uint32_t G, uint32_t k, uint32_t sms, uint32_t* scratch,
                                uint64_t* tmp, uint64_t* out, uint32_t* bucket_off, uint32_t* inst, cudaStream_t s);
 // cluster == 0: tables in the global arena; 1: one CTA's shared memory; >1: a cluster's.
 cudaError_t launch_subgraphs(const SubgraphArgs& a, int words, uint32_t cluster, uint32_t threads, cudaStream_t s);
