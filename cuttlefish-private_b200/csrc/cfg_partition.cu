@@ -20,7 +20,6 @@ namespace {
 
 constexpr int WARPS_PER_BLOCK = 8;
 constexpr uint32_t STAGE = 256;       // records a warp gathers in shared memory per reservation
-constexpr uint32_t MODW = 160;        // residues kept: the cut test indexes up to w - 1 + 32
 
 __device__ __forceinline__ uint32_t lanemask_lt() { uint32_t m; asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m)); return m; }
 
@@ -84,7 +83,6 @@ __device__ __forceinline__ uint64_t min64(uint64_t a, uint64_t b) { return a < b
 
 // Processes the (k-1)-mer positions [j0, j1) of one fragment: emits every weak
 // super k-mer whose run starts there.
-// mod_w[x] = x % w for x < MODW (w <= 126): the cap-cut test without a division.
 // hist: this fragment's job's histogram (the run's, or its job's slice of a batch's);
 // nullptr when the bucket sort counts the records itself.
 //
@@ -98,8 +96,8 @@ __device__ __forceinline__ uint64_t min64(uint64_t a, uint64_t b) { return a < b
 // O(log w) work per position, no shared memory.  For w >= 96 (E = 6, dq = w - 64 > 32)
 // the second block starts two chunks back: level E of the chunk before the previous is kept.
 template <int E>
-__device__ void sweep_fragment(const PartitionArgs& a, const uint8_t* mod_w, uint64_t F0, uint32_t FL,
-                               uint32_t j0, uint32_t j1, unsigned long long* hist, Stage& st) {
+__device__ void sweep_fragment(const PartitionArgs& a, uint64_t F0, uint32_t FL, uint32_t j0, uint32_t j1,
+                               unsigned long long* hist, Stage& st) {
     const uint32_t lane = threadIdx.x & 31;
     const uint32_t k = a.k, l = a.l, w = a.w;
     const uint32_t M = FL - k + 2;                 // (k-1)-mers in the fragment
@@ -134,9 +132,13 @@ __device__ void sweep_fragment(const PartitionArgs& a, const uint8_t* mod_w, uin
     // `start`, ceil((w - 1) / 32) chunks (at least one)
     for (int c = (int)max(1u, (w - 1 + 31) / 32); c >= 1; --c) levels(hash_at((int64_t)start - 32 * c + w - 1 + lane));
 
+    // Every change of g is a cut, so from a cut to the next one g is the same: a piece's g is that
+    // of the position before the cut that ends it, and its start's "change" bit is in the mask.
     bool active = false;
-    uint32_t r0 = 0, last_cut = 0, last_cut_g = 0, last_cut_chg = 0, carry_g = 0;
-    uint32_t carry_rem = 0;   // (base - start of the run in progress) % w
+    uint32_t last_cut = 0, last_cut_chg = 0;
+    uint32_t carry_g = ~0u;   // g of the position before base (none at the fragment's start: a change)
+    uint32_t carry_d = 0;     // base - start of the run in progress
+    const uint32_t lt = lanemask_lt(), inside = min(M, j1);
 
     // each chunk's new l-mer hash is computed one chunk ahead, so its loads and
     // multiplies overlap the window minima of the chunk before
@@ -146,97 +148,92 @@ __device__ void sweep_fragment(const PartitionArgs& a, const uint8_t* mod_w, uin
         h_next = hash_at((int64_t)base + 32 + w - 1 + lane);
         const uint64_t m = levels(h);
         const uint32_t j = base + lane;
-        const bool valid = j < M;
-        const uint32_t g = valid ? (uint32_t)m & a.gmask : 0u;
+        const bool interior = base >= j0 && base + 32 <= inside;   // uniform: every position is one of [j0, j1)
+        uint32_t g = (uint32_t)m & a.gmask;
+        if (!interior && j >= M) g = 0;
         uint32_t gprev = __shfl_up_sync(0xffffffffu, g, 1);
         if (lane == 0) gprev = carry_g;
-        const bool is_chg = valid && j >= j0 && (j == 0 || gprev != g);
+        const bool is_chg = gprev != g && (interior || (j < M && j >= j0));
         const uint32_t chg = __ballot_sync(0xffffffffu, is_chg);
 
-        bool just_activated = false;
-        uint32_t r0_lane = 0;
+        uint32_t act = 0xffffffffu, first = 0;   // positions of runs that start in [j0, j1); the first run's start
         if (!active) {
             if (chg == 0) {
                 if (base + 32 >= j1 || base + 32 >= M) return;   // no run starts in [j0, j1)
                 carry_g = __shfl_sync(0xffffffffu, g, 31);
                 continue;
             }
-            r0_lane = __ffs(chg) - 1;
-            r0 = base + r0_lane;
-            if (r0 >= j1) return;
-            active = true; just_activated = true;
-            last_cut = r0;
-            last_cut_g = __shfl_sync(0xffffffffu, g, r0_lane);
+            const uint32_t r0_lane = __ffs(chg) - 1;
+            if (base + r0_lane >= j1) return;
+            active = true;
+            first = 1u << r0_lane;
+            act = 0xffffffffu << r0_lane;
+            last_cut = base + r0_lane;
             last_cut_chg = 1;
         }
-        const uint32_t act_mask = just_activated ? (0xffffffffu << r0_lane) : 0xffffffffu;
 
-        // run start of each position: highest change at or below it, else the carried one
-        const uint32_t le = chg & (lanemask_lt() | (1u << lane));
-        const uint32_t rem = le ? mod_w[lane - (31 - __clz(le))] : mod_w[carry_rem + lane];
-        const bool is_cut = valid && ((act_mask >> lane) & 1) && (is_chg || rem == 0);
-        uint32_t cut = __ballot_sync(0xffffffffu, is_cut);
+        // distance to the start of the position's run: from the highest change at or below it,
+        // else carried; a run is cut again every w positions, which a minimizer seldom reaches
+        const uint32_t le = chg & (lt | (1u << lane));
+        const uint32_t d = le ? lane - (31 - __clz(le)) : carry_d + lane;
+        uint32_t cut = chg & act;
+        if (__any_sync(0xffffffffu, d >= w && ((act >> lane) & 1)))
+            cut = __ballot_sync(0xffffffffu, ((act >> lane) & 1) && (interior || j < M) && d % w == 0);
 
         // stop at the first change at or past j1: the run it starts belongs to the next segment
         bool stopping = false;
-        {
-            const uint32_t past = __ballot_sync(0xffffffffu, valid && j >= j1);
-            const uint32_t stop = chg & past;
+        if (base + 32 > j1) {
+            const uint32_t stop = chg & __ballot_sync(0xffffffffu, j >= j1);   // (a change is a valid position)
             if (stop) {
                 const uint32_t sl = __ffs(stop) - 1;
                 cut &= (sl == 31) ? 0xffffffffu : ((2u << sl) - 1);
                 stopping = true;
             }
         }
-        uint32_t emit = cut;
-        if (just_activated) emit &= ~(1u << r0_lane);
-
-        // piece [c, c') ends at every emitting lane c' = j
-        const uint32_t below = cut & lanemask_lt();
-        const uint32_t pl = below ? (31 - __clz(below)) : 0;
-        const uint32_t pg = __shfl_sync(0xffffffffu, g, pl);
-        const uint32_t pchg = __shfl_sync(0xffffffffu, (uint32_t)is_chg, pl);
+        const uint32_t emit = cut & ~first;   // piece [c, c') ends at every emitting lane c' = j
         const bool fin = !stopping && (base + 32 >= M);      // the fragment's last (k-1)-mer is in this chunk
         const uint32_t n_emit = __popc(emit) + (fin ? 1 : 0);
         if (st.n + n_emit > STAGE) stage_flush(a, st);
         const uint32_t slot0 = st.n;
         st.n += n_emit;
         if ((emit >> lane) & 1) {
+            const uint32_t below = cut & lt, pl = 31 - __clz(below);
             const uint32_t c = below ? base + pl : last_cut;
-            const uint32_t cg = below ? pg : last_cut_g;
-            const uint32_t cchg = below ? pchg : last_cut_chg;
+            const uint32_t cchg = below ? (chg >> pl) & 1u : last_cut_chg;
             const uint32_t lj = c > 0;
             const uint32_t len = lj + (j - c + k - 2) + 1;
-            const uint64_t r = rec_pack((uint32_t)(F0 + c - lj), len, lj & cchg, is_chg ? 1u : 0u, cg);
-            st.buf[slot0 + __popc(emit & lanemask_lt())] = r;
-            if (hist) atomicAdd(hist + cg, 1ull | ((unsigned long long)(len - k + 1) << 32));
+            const uint64_t r = rec_pack((uint32_t)(F0 + c - lj), len, lj & cchg, is_chg ? 1u : 0u, gprev);
+            st.buf[slot0 + __popc(emit & lt)] = r;
+            if (hist) atomicAdd(hist + gprev, 1ull | ((unsigned long long)(len - k + 1) << 32));
         }
         // carries: last cut / run start of this chunk
         if (cut) {
             const uint32_t hl = 31 - __clz(cut);
             last_cut = base + hl;
-            last_cut_g = __shfl_sync(0xffffffffu, g, hl);
-            last_cut_chg = __shfl_sync(0xffffffffu, (uint32_t)is_chg, hl);
+            last_cut_chg = (chg >> hl) & 1u;
         }
-        carry_rem = chg ? mod_w[32 - (31 - __clz(chg))] : mod_w[carry_rem + 32];
-        carry_g = __shfl_sync(0xffffffffu, g, 31);
-        if (fin && lane == 0) {   // final piece [last_cut, M): not joined on the right
-            const uint32_t c = last_cut, lj = c > 0;
-            const uint32_t len = lj + (FL - c);
-            const uint64_t r = rec_pack((uint32_t)(F0 + c - lj), len, lj & last_cut_chg, 0, last_cut_g);
-            st.buf[slot0 + __popc(emit)] = r;
-            if (hist) atomicAdd(hist + last_cut_g, 1ull | ((unsigned long long)(len - k + 1) << 32));
+        if (fin) {   // final piece [last_cut, M): not joined on the right
+            const uint32_t gl = __shfl_sync(0xffffffffu, g, M - 1 - base);
+            if (lane == 0) {
+                const uint32_t c = last_cut, lj = c > 0;
+                const uint32_t len = lj + (FL - c);
+                const uint64_t r = rec_pack((uint32_t)(F0 + c - lj), len, lj & last_cut_chg, 0, gl);
+                st.buf[slot0 + __popc(emit)] = r;
+                if (hist) atomicAdd(hist + gl, 1ull | ((unsigned long long)(len - k + 1) << 32));
+            }
         }
         if (stopping || fin) return;
+        carry_d = chg ? 32 - (31 - __clz(chg)) : carry_d + 32;
+        carry_g = __shfl_sync(0xffffffffu, g, 31);
     }
 }
 
+// Four CTAs per SM (64 registers) for 32 <= w < 64, where the compiler's own choice is 96
+// registers and two CTAs: 300 Mbp at k = 63 4.49 -> 3.98 ms.  The other depths are faster left
+// at their 62 to 80 registers, three CTAs (k = 31: 3.56 ms, 3.71 at 64 registers).
 template <int E>
-__global__ void __launch_bounds__(WARPS_PER_BLOCK * 32) k_partition(const PartitionArgs a) {
+__global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, E == 5 ? 4 : 0) k_partition(const PartitionArgs a) {
     __shared__ uint64_t stages[WARPS_PER_BLOCK][STAGE];
-    __shared__ uint8_t mod_w[MODW];
-    if (threadIdx.x < MODW) mod_w[threadIdx.x] = (uint8_t)(threadIdx.x % a.w);
-    __syncthreads();
     Stage st{stages[threadIdx.x >> 5], 0};
     // this launch's bases and fragments (the fragment table is read only inside them:
     // the entries of other pieces may not have landed yet)
@@ -267,7 +264,7 @@ __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32) k_partition(const Partit
             const uint32_t j0 = s0 > F0 ? (uint32_t)(s0 - F0) : 0;
             const uint64_t e = s1 - F0;
             const uint32_t j1 = e < M ? (uint32_t)e : M;
-            if (j0 < j1) sweep_fragment<E>(a, mod_w, F0, FL, j0, j1,
+            if (j0 < j1) sweep_fragment<E>(a, F0, FL, j0, j1,
                                           a.hist ? a.hist + (a.frag_gbase ? a.frag_gbase[f] : 0u) : nullptr, st);
         }
     }
