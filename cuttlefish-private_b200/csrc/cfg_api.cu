@@ -31,7 +31,10 @@ struct cfg_ctx {
     DevBuf packed, frag_off, frag_len, text;
     // cfg_submit_packed copies the input in pieces on its own stream; the partition of a
     // piece waits only for that piece's copies (no pieces: the input is already resident)
-    static constexpr int MAX_PIECES = 8;
+    // (a call on 500 Mbp, k = 63, in 8, 4, 2, 1 pieces: 116.4 115.5 115.1 115.1 ms; 100 Mbp, k = 31:
+    // 39.3 38.2 37.9 37.7; 3 M reads, whose fragment table outweighs their bases: 19.4 18.9 20.0
+    // 22.1 -- every piece is a launch with a tail of its own)
+    static constexpr int MAX_PIECES = 4;
     struct Piece { uint64_t f0, f1, b0, b1; };
     std::vector<Piece> pieces;
     cudaStream_t copy_stream = nullptr;
