@@ -414,13 +414,20 @@ __device__ __forceinline__ Res reserve_block(const Sink& sk, Block& B, unsigned 
     }
     if (lane == 31) { B.rs[0][wid] = a; B.rs[1][wid] = b; B.rs[2][wid] = c; }
     __syncthreads();
-    if (threadIdx.x < 3) {   // thread q: kind q's warp totals into offsets, one atomic
-        unsigned long long* r = B.rs[threadIdx.x];
-        unsigned long long run = 0;
-        for (uint32_t w = 0; w < nw; ++w) { const unsigned long long t = r[w]; r[w] = run; run += t; }
-        unsigned long long* cur = threadIdx.x == 0 ? sk.fasta_cur : threadIdx.x == 1 ? sk.lm_cur : sk.lm_text_cur;
-        const unsigned long long base = run ? atomicAdd(cur, run) : 0ull;
-        for (uint32_t w = 0; w < nw; ++w) r[w] += base;
+    for (uint32_t q = wid; q < 3; q += nw) {   // warp q: kind q's warp totals into offsets, one atomic
+        unsigned long long* r = B.rs[q];
+        const unsigned long long own = lane < nw ? r[lane] : 0ull;
+        unsigned long long x = own;
+#pragma unroll
+        for (int d = 1; d < 32; d <<= 1) {
+            const unsigned long long y = __shfl_up_sync(FULL, x, d);
+            if (lane >= (uint32_t)d) x += y;
+        }
+        const unsigned long long total = __shfl_sync(FULL, x, 31);
+        unsigned long long base = 0;
+        if (lane == 0 && total) base = atomicAdd(q == 0 ? sk.fasta_cur : q == 1 ? sk.lm_cur : sk.lm_text_cur, total);
+        base = __shfl_sync(FULL, base, 0);
+        if (lane < nw) r[lane] = base + x - own;
     }
     __syncthreads();
     const Res out{B.rs[0][wid] + a - fa, B.rs[1][wid] + b - nlm, B.rs[2][wid] + c - lmb};
