@@ -165,7 +165,8 @@ int run_partition(cfg_ctx* c) {
         a.err = &dev_words(c)->err;
         const uint64_t n_words = (c->n_bases + 31) / 32;
         if (!c->rcw.ensure(8 * (n_words + 4))) return fail(c, CFG_ERR_OOM, "reverse-complement words");
-        a.rcw = c->rcw.as<uint64_t>();
+        uint64_t* const rcw = c->rcw.as<uint64_t>() + 1;   // one readable word before the first
+        a.rcw = rcw;
         CK(cudaEventRecord(c->ev[1], c->stream));
         // input still in flight: a launch per piece as it lands; all landed: one launch
         bool landed = c->pieces.empty();
@@ -175,7 +176,7 @@ int run_partition(cfg_ctx* c) {
             landed = q == cudaSuccess;
         }
         if (landed) {
-            launch_rc_words(c->d_packed, 0, n_words, c->rcw.as<uint64_t>(), c->stream);
+            launch_rc_words(c->d_packed, 0, n_words, rcw, c->stream);
             launch_partition(a, c->stream);
             c->launches += 2;
         } else {   // each piece of the input as soon as its copies have landed
@@ -183,7 +184,7 @@ int run_partition(cfg_ctx* c) {
                 const cfg_ctx::Piece& pc = c->pieces[i];
                 CK(cudaStreamWaitEvent(c->stream, c->piece_ev[i], 0));
                 a.base0 = pc.b0; a.base1 = pc.b1; a.frag_lo = pc.f0; a.frag_hi = pc.f1;
-                launch_rc_words(c->d_packed, pc.b0 >> 5, (pc.b1 + 31) >> 5, c->rcw.as<uint64_t>(), c->stream);
+                launch_rc_words(c->d_packed, pc.b0 >> 5, (pc.b1 + 31) >> 5, rcw, c->stream);
                 launch_partition(a, c->stream);
                 c->launches += 2;
             }

@@ -45,12 +45,6 @@ __device__ __forceinline__ uint64_t rc_word(uint64_t x, uint32_t n) {
     return n == 0 ? 0 : (r >> (64 - 2 * n));
 }
 
-// min(hash(lmer), hash(rc(lmer))) -- Min_Iterator::lmer_hash (include/Minimizer_Iterator.hpp:291-296)
-__device__ __forceinline__ uint64_t lmer_hash(uint64_t lmer, uint32_t l, uint64_t seed0) {
-    const uint64_t a = wyhash8(lmer, seed0), b = wyhash8(rc_word(lmer, l), seed0);
-    return a < b ? a : b;
-}
-
 // 64 bases starting at stream position p, base p at bits 63:62 (needs 2 words of padding).
 __device__ __forceinline__ uint64_t window64(const uint64_t* __restrict__ s, uint64_t p) {
     const uint64_t w = p >> 5;

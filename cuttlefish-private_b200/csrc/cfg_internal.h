@@ -64,8 +64,9 @@ struct PartitionArgs {
     // job whose input arrives in pieces partitions each piece as soon as it has landed.
     uint64_t base0, base1, frag_lo, frag_hi;
     // every packed word reverse-complemented in place (its 32 bases reversed, each
-    // complemented), written by launch_rc_words for this launch's words; nullptr: each
-    // l-mer's reverse complement is computed from the l-mer itself
+    // complemented), written by launch_rc_words for this launch's words, with one readable
+    // word before the first; nullptr: each l-mer's reverse complement is computed from the
+    // l-mer itself
     const uint64_t* rcw;
 };
 // Stream bases per warp of a partition launch.  A warp walks its segment 32 bases at a

@@ -23,26 +23,39 @@ constexpr uint32_t STAGE = 256;       // records a warp gathers in shared memory
 
 __device__ __forceinline__ uint32_t lanemask_lt() { uint32_t m; asm("mov.u32 %0, %%lanemask_lt;" : "=r"(m)); return m; }
 
-__device__ __forceinline__ uint64_t lmer_at(const uint64_t* __restrict__ s, uint64_t p, uint32_t l) {
-    return window64(s, p) >> (64 - 2 * l);
-}
-
-// min(hash(l-mer at p), hash(its reverse complement)).  With the reverse-complemented
-// words at hand, the reverse complement is a second window: its first base is the
-// l-mer's last, e = p + l - 1, at index 31 - (e mod 32) of rcw[e / 32], and it continues
-// into rcw[e / 32 - 1] -- two loads and a funnel shift instead of a bit reversal per
-// l-mer (this kernel is bound by the integer ALU pipe, not by loads).
-__device__ __forceinline__ uint64_t lmer_hash_at(const PartitionArgs& a, uint64_t p, uint32_t l) {
-    const uint64_t fw = lmer_at(a.packed, p, l);
-    if (!a.rcw) return lmer_hash(fw, l, a.seed0);
-    const uint64_t e = p + l - 1, w2 = e >> 5;
-    const uint32_t j = 31 - (uint32_t)(e & 31);
-    const uint64_t hi = __ldg(a.rcw + w2);
-    const uint64_t win = j == 0 ? hi : (hi << (2 * j)) | (w2 ? __ldg(a.rcw + w2 - 1) >> (64 - 2 * j) : 0ull);
-    const uint64_t rc = win >> (64 - 2 * l);
-    const uint64_t x = wyhash8(fw, a.seed0), y = wyhash8(rc, a.seed0);
-    return x < y ? x : y;
-}
+// A lane's l-mers of one fragment, one every 32 positions: min(hash(l-mer), hash(its reverse
+// complement)), Min_Iterator::lmer_hash (include/Minimizer_Iterator.hpp:291-296).  A step moves
+// the lane by one packed word and leaves its bit offsets as they are, so addresses and shifts
+// are worked out once per fragment: this kernel is bound by the integer ALU pipe, not by loads
+// (300 Mbp at k = 31, 3.56 -> 3.43 ms against working them out per l-mer; 150-base reads 3.89
+// -> 3.82, 101-base reads at k = 27 1.49 -> 1.39 per 101 Mbp; k = 63 the same).
+// With the reverse-complemented words at hand, the reverse complement is a second window: its
+// first base is the l-mer's last, e = p + l - 1, at index 31 - (e mod 32) of rcw[e / 32], and it
+// continues into rcw[e / 32 - 1].  Both windows always read their second word, the padding
+// word after the stream's last (before rcw's first) where the l-mer needs no bit of it; a
+// lane whose l-mer lies outside the fragment reads nothing and gets "none", all ones.
+struct LmerWalk {
+    const uint64_t *f, *r;    // the word of the l-mer's first base; of rcw, of its last
+    uint32_t sf, sr;          // bits before the l-mer in its word; before its reverse complement in rcw's
+    __device__ __forceinline__ LmerWalk(const PartitionArgs& a, int64_t p) {
+        f = a.packed + (p >> 5); sf = 2 * (uint32_t)(p & 31);
+        const int64_t e = p + a.l - 1;
+        r = a.rcw + (e >> 5); sr = 62 - 2 * (uint32_t)(e & 31);
+    }
+    __device__ __forceinline__ uint64_t next(const PartitionArgs& a, bool valid) {
+        uint64_t h = ~0ull;
+        if (valid) {
+            const uint32_t top = 64 - 2 * a.l;
+            const uint64_t fw = ((__ldg(f) << sf) | ((__ldg(f + 1) >> 1) >> (63 - sf))) >> top;
+            const uint64_t rc = a.rcw ? ((__ldg(r) << sr) | ((__ldg(r - 1) >> 1) >> (63 - sr))) >> top
+                                      : rc_word(fw, a.l);
+            const uint64_t x = wyhash8(fw, a.seed0), y = wyhash8(rc, a.seed0);
+            h = x < y ? x : y;
+        }
+        ++f; ++r;
+        return h;
+    }
+};
 
 __global__ void k_rc_words(const uint64_t* __restrict__ packed, uint64_t w0, uint64_t w1, uint64_t* rcw) {
     for (uint64_t w = w0 + (uint64_t)blockIdx.x * blockDim.x + threadIdx.x; w < w1; w += (uint64_t)gridDim.x * blockDim.x) {
@@ -104,10 +117,6 @@ __device__ void sweep_fragment(const PartitionArgs& a, uint64_t F0, uint32_t FL,
     const uint32_t n_lmers = FL - l + 1;
     const uint32_t start = j0 == 0 ? 0 : j0 - 1;   // position j0-1 only primes the change test
     const uint32_t dq = w - (1u << E);
-    // hash of l-mer q, or "none" (all ones, above every hash) outside the fragment
-    auto hash_at = [&](int64_t q) -> uint64_t {   // a negative q wraps above every l-mer count: one compare
-        return (uint64_t)q < (uint64_t)n_lmers ? lmer_hash_at(a, F0 + (uint64_t)q, l) : ~0ull;
-    };
     uint64_t lv[E + 1], pv[E + 1];   // this chunk's / the previous chunk's level values
     uint64_t ppE = ~0ull;            // level E two chunks back (E = 6 only)
 #pragma unroll
@@ -130,7 +139,11 @@ __device__ void sweep_fragment(const PartitionArgs& a, uint64_t F0, uint32_t FL,
     };
     // prime the levels with the chunks before the first: their hashes reach back to l-mer
     // `start`, ceil((w - 1) / 32) chunks (at least one)
-    for (int c = (int)max(1u, (w - 1 + 31) / 32); c >= 1; --c) levels(hash_at((int64_t)start - 32 * c + w - 1 + lane));
+    const int n_prime = (int)max(1u, (w - 1 + 31) / 32);
+    const int64_t q0 = (int64_t)start + w - 1 + lane;   // the lane's l-mer in the first chunk
+    LmerWalk lm(a, (int64_t)F0 + q0 - 32 * n_prime);
+    for (int c = n_prime; c >= 1; --c) levels(lm.next(a, (uint64_t)(q0 - 32 * c) < (uint64_t)n_lmers));
+    uint32_t left = q0 < (int64_t)n_lmers ? (uint32_t)(n_lmers - q0) : 0u;   // l-mers from the lane's next one to the end
 
     // Every change of g is a cut, so from a cut to the next one g is the same: a piece's g is that
     // of the position before the cut that ends it, and its start's "change" bit is in the mask.
@@ -142,10 +155,11 @@ __device__ void sweep_fragment(const PartitionArgs& a, uint64_t F0, uint32_t FL,
 
     // each chunk's new l-mer hash is computed one chunk ahead, so its loads and
     // multiplies overlap the window minima of the chunk before
-    uint64_t h_next = hash_at((int64_t)start + w - 1 + lane);
+    uint64_t h_next = lm.next(a, left > 0);
     for (uint32_t base = start;; base += 32) {
         const uint64_t h = h_next;
-        h_next = hash_at((int64_t)base + 32 + w - 1 + lane);
+        left = left > 32 ? left - 32 : 0u;
+        h_next = lm.next(a, left > 0);
         const uint64_t m = levels(h);
         const uint32_t j = base + lane;
         const bool interior = base >= j0 && base + 32 <= inside;   // uniform: every position is one of [j0, j1)
@@ -230,7 +244,7 @@ __device__ void sweep_fragment(const PartitionArgs& a, uint64_t F0, uint32_t FL,
 
 // Four CTAs per SM (64 registers) for 32 <= w < 64, where the compiler's own choice is 96
 // registers and two CTAs: 300 Mbp at k = 63 4.49 -> 3.98 ms.  The other depths are faster left
-// at their 62 to 80 registers, three CTAs (k = 31: 3.56 ms, 3.71 at 64 registers).
+// at their 62 to 80 registers, three CTAs (k = 31: 3.43 ms at three CTAs; at 64 registers it lost 4 %).
 template <int E>
 __global__ void __launch_bounds__(WARPS_PER_BLOCK * 32, E == 5 ? 4 : 0) k_partition(const PartitionArgs a) {
     __shared__ uint64_t stages[WARPS_PER_BLOCK][STAGE];
