@@ -11,9 +11,10 @@
 //      super-bucket, and the slab is then moved tile by tile: a tile is counting-sorted
 //      by super-bucket in shared memory and written out as contiguous runs;
 //   2. one CTA per super-bucket sorts its records by the low bits of g inside their
-//      region (a few MB, L2-resident), counting records and k-mer instances per
-//      subgraph in shared memory: the bucket offsets and instance counts the subgraph
-//      kernels and the host planning read come out of this pass.
+//      region, counting records and k-mer instances per subgraph in shared memory: the
+//      bucket offsets and instance counts the subgraph kernels and the plan read come out
+//      of this pass.  It goes tile by tile through shared memory as well: records written
+//      one by one to their subgraph's place cost a 32-byte sector each.
 // The order of records inside a bucket is not stable (nothing downstream depends on it:
 // the vertex states are order-independent and first occurrences are stream positions).
 #include "cfg_internal.h"
@@ -23,10 +24,12 @@ namespace cfg {
 namespace {
 
 constexpr uint32_t SB_THREADS = 512;
+constexpr uint32_t COUNT_THREADS = 1024;
 constexpr uint32_t SB_TILE = 8192;        // records per pass-1 tile (64 KB of shared memory)
 constexpr uint32_t SB_MAX_BINS = 1024;    // super-buckets, and subgraphs per super-bucket
 constexpr uint32_t SCAN_ITEMS = 8192;     // entries per CTA of the (super-bucket, slab) scan
 constexpr uint32_t UNROLL = 8;            // record loads in flight per thread (a record is never all ones)
+constexpr uint32_t LO_TILE = UNROLL * SB_THREADS;   // records per pass-2 tile (32 KB)
 
 // The record count is a device word, so the sort is queued behind the partition without a
 // wait; a count past the buffer (the partition overflowed and is rerun) sorts nothing.
@@ -65,8 +68,9 @@ __device__ void smem_excl_scan(uint32_t* bins, uint32_t nb, uint32_t* warp_sums,
     __syncthreads();
 }
 
-// Pass 1a: counts[h * S + s] = records of slab s in super-bucket h.
-__global__ void __launch_bounds__(SB_THREADS) k_sb_count(const uint64_t* __restrict__ flat, RecCount nr, uint32_t lbits,
+// Pass 1a: counts[h * S + s] = records of slab s in super-bucket h.  One CTA per SM, so it
+// takes 1024 threads to keep enough loads in flight (0.1 ms less for 210 M records than 512).
+__global__ void __launch_bounds__(COUNT_THREADS) k_sb_count(const uint64_t* __restrict__ flat, RecCount nr, uint32_t lbits,
                                                          uint32_t H, uint32_t* __restrict__ counts) {
     __shared__ uint32_t cnt[SB_MAX_BINS];
     const uint32_t S = gridDim.x, s = blockIdx.x;
@@ -226,16 +230,24 @@ __global__ void __launch_bounds__(SB_THREADS) k_sb_move_hi(const uint64_t* __res
 
 // Pass 2: super-bucket h = [base_h, base_{h+1}) of tmp sorted by the low bits of g into
 // out; bucket offsets and k-mer instance counts per subgraph.
-__global__ void __launch_bounds__(SB_THREADS) k_sb_move_lo(const uint64_t* __restrict__ tmp, RecCount nr, uint32_t lbits,
+// A tile is counting-sorted in shared memory and written as runs (32 records a subgraph at 128
+// subgraphs per super-bucket).  Written record by record the pass was bound by the L2's sector
+// writes: the whole sort of 10 M reads' 210 M records 3.71 -> 2.75 ms, of 22 M records over
+// 524288 subgraphs 0.49 -> 0.36, of 42 M over 32768 0.62 -> 0.58.  A super-bucket of one tile or
+// less is written record by record: 813 records each, the sort takes 46 us so and 50 us
+// through a tile.  Three CTAs per SM (40 registers); at four, with a few spills, 2.90 ms.
+__global__ void __launch_bounds__(SB_THREADS, 3) k_sb_move_lo(const uint64_t* __restrict__ tmp, RecCount nr, uint32_t lbits,
                                                            uint32_t H, uint32_t S, const uint32_t* __restrict__ counts,
                                                            uint32_t k, uint64_t* __restrict__ out,
                                                            uint32_t* __restrict__ bucket_off, uint32_t* __restrict__ inst) {
+    __shared__ uint64_t stage[LO_TILE];
     __shared__ uint32_t cnt[SB_MAX_BINS], ins[SB_MAX_BINS], fill[SB_MAX_BINS];
+    uint32_t* const tcnt = ins;   // once ins is written out: a tile's counts, then its offsets
     __shared__ uint32_t ws[SB_THREADS / 32 + 1];
     const uint32_t h = blockIdx.x, L = 1u << lbits, lmask = L - 1;
     const uint64_t n = records(nr);
     const uint64_t a = counts[(uint64_t)h * S], b = h + 1 < H ? counts[(uint64_t)(h + 1) * S] : n;
-    for (uint32_t l = threadIdx.x; l < L; l += blockDim.x) { cnt[l] = 0; ins[l] = 0; fill[l] = 0; }
+    for (uint32_t l = threadIdx.x; l < L; l += blockDim.x) { cnt[l] = 0; ins[l] = 0; }
     __syncthreads();
     for (uint64_t i0 = a + threadIdx.x; i0 < b; i0 += (uint64_t)UNROLL * blockDim.x) {
         uint64_t r[UNROLL];
@@ -259,19 +271,43 @@ __global__ void __launch_bounds__(SB_THREADS) k_sb_move_lo(const uint64_t* __res
         inst[((uint64_t)h << lbits) + l] = ins[l];
     }
     if (h == H - 1 && threadIdx.x == 0) bucket_off[(uint64_t)H << lbits] = (uint32_t)n;
-    for (uint64_t i0 = a + threadIdx.x; i0 < b; i0 += (uint64_t)UNROLL * blockDim.x) {
+    __syncthreads();   // ins is read above before the tiles use it
+    for (uint32_t l = threadIdx.x; l < L; l += SB_THREADS) fill[l] = cnt[l];
+    if (b - a <= LO_TILE) {   // one tile: straight to its places, a few KB that the L2 holds
+        __syncthreads();
+        for (uint64_t i = a + threadIdx.x; i < b; i += SB_THREADS) {
+            const uint64_t x = tmp[i];
+            out[a + atomicAdd(&fill[rec_g(x) & lmask], 1u)] = x;
+        }
+        return;
+    }
+    for (uint64_t t0 = a; t0 < b; t0 += LO_TILE) {
+        const uint32_t tn = (uint32_t)(b - t0 < LO_TILE ? b - t0 : LO_TILE);
         uint64_t r[UNROLL];
+        uint32_t rank[UNROLL];
 #pragma unroll
         for (uint32_t j = 0; j < UNROLL; ++j) {
-            const uint64_t i = i0 + (uint64_t)j * blockDim.x;
-            r[j] = i < b ? tmp[i] : ~0ull;
+            const uint32_t i = j * SB_THREADS + threadIdx.x;
+            r[j] = i < tn ? tmp[t0 + i] : ~0ull;
         }
+        for (uint32_t l = threadIdx.x; l < L; l += SB_THREADS) tcnt[l] = 0;
+        __syncthreads();
+#pragma unroll
+        for (uint32_t j = 0; j < UNROLL; ++j) rank[j] = r[j] != ~0ull ? atomicAdd(&tcnt[rec_g(r[j]) & lmask], 1u) : 0u;
+        __syncthreads();
+        smem_excl_scan(tcnt, L, ws, ws + SB_THREADS / 32);   // tcnt: tile offsets per subgraph
 #pragma unroll
         for (uint32_t j = 0; j < UNROLL; ++j)
-            if (r[j] != ~0ull) {
-                const uint32_t l = rec_g(r[j]) & lmask;
-                out[a + cnt[l] + atomicAdd(&fill[l], 1u)] = r[j];
-            }
+            if (r[j] != ~0ull) stage[tcnt[rec_g(r[j]) & lmask] + rank[j]] = r[j];
+        __syncthreads();
+        for (uint32_t i = threadIdx.x; i < tn; i += SB_THREADS) {
+            const uint64_t x = stage[i];
+            const uint32_t l = rec_g(x) & lmask;
+            out[a + fill[l] + (i - tcnt[l])] = x;
+        }
+        __syncthreads();
+        for (uint32_t l = threadIdx.x; l < L; l += SB_THREADS) fill[l] += (l + 1 < L ? tcnt[l + 1] : tn) - tcnt[l];
+        __syncthreads();   // tcnt is read above before the next tile clears it
     }
 }
 
@@ -295,7 +331,7 @@ cudaError_t launch_bucket_sort(const uint64_t* flat, const unsigned long long* n
     uint32_t* sums = scratch + m;
     const uint32_t nsums = (uint32_t)((m + SCAN_ITEMS - 1) / SCAN_ITEMS);
     const RecCount n{n_dev, cap};
-    k_sb_count<<<S, SB_THREADS, 0, s>>>(flat, n, lbits, H, counts);
+    k_sb_count<<<S, COUNT_THREADS, 0, s>>>(flat, n, lbits, H, counts);
     k_sb_scan_sums<<<nsums, SB_THREADS, 0, s>>>(counts, m, sums);
     k_sb_scan_apply<<<nsums, SB_THREADS, 0, s>>>(counts, m, sums, nsums);
     const size_t smem = 2 * SB_TILE * 8 + 2 * SB_MAX_BINS * 4 + (SB_THREADS / 32 + 1) * 4;

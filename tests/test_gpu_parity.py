@@ -274,3 +274,23 @@ def test_table_shapes(k):
         line = s // 2 if k == 31 else 2 * s // 3          # k-mer instances that still fit
         for n in (line * 9 // 10, line, line + line // 8 + 1):
             compare([synth.random_seq(rng, n + k - 1)], k, 20, 1, 1)
+
+
+@pytest.mark.parametrize("n,length,G", [(4095, 60, 16384), (4096, 60, 16384), (4097, 60, 16384), (12301, 60, 32768),
+                                        (1501, 3000, 131072)])
+def test_bucket_sort_tiles(n, length, G):
+    """Copies of one sequence: every super-bucket holds a multiple of n records, to either side of a tile of the sort's
+    second pass (4096 records), and at 3000 bases several subgraphs to a super-bucket."""
+    records = [synth.random_seq(np.random.default_rng(70), length)] * n
+    o = orc.OracleRun(records, 31, 20, 1, G)
+    counts, rec_ms, st, fa, lm = gpu_run(records, 31, 20, 1, G)
+
+    def dumped(rows):   # the dumps hold a subgraph's low 16 bits
+        out = collections.Counter()
+        for (g, *rest), m in rows.items():
+            out[(g & 0xFFFF, *rest)] += m
+        return out
+    assert counts.n_records == o.counts["n_records"] and counts.n_instances == o.counts["n_instances"]
+    assert rec_ms == dumped(o.records), "weak super k-mer records differ"
+    assert {(g & 0xFFFF, key): s for (g, key), s in st.items()} == {(g & 0xFFFF, key): s for (g, key), s in o.states.items()}
+    assert fa == o.fasta_records() and lm == dumped(o.lmtigs)
