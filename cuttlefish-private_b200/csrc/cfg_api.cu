@@ -4,6 +4,7 @@
 #include "cfg_device.cuh"
 #include "cfg_host.h"
 #include "cfg_internal.h"
+#include "cfg_sides.h"
 
 #include <algorithm>
 #include <cstdio>
@@ -39,11 +40,7 @@ struct cfg_ctx {
     std::vector<Piece> pieces;
     cudaStream_t copy_stream = nullptr;
     cudaEvent_t piece_ev[MAX_PIECES] = {}, idle_ev = nullptr;
-    // table classes of one pass run side by side (see launch_planned): streams, and the events
-    // that start them after, and join them to, the context's stream
-    static constexpr int SIDES = 3;
-    cudaStream_t side[SIDES] = {};
-    cudaEvent_t fork_ev = nullptr, join_ev[SIDES] = {};
+    SideStreams sides;   // table classes of one pass run side by side (see launch_planned)
     ParseBuffers parse;
     // cfg_submit_text: events before and after the text's copy and after the parse
     cudaEvent_t text_ev[3] = {};
@@ -254,12 +251,11 @@ int ensure_arena(cfg_ctx* c, uint64_t slots) {
     return CFG_OK;
 }
 
-int launch_classes(cfg_ctx* c, const RunWords& w, uint32_t& sides) {
+int launch_classes(cfg_ctx* c, const RunWords& w) {
     const PlanArgs pa = plan_args(c);
     uint32_t n_shapes = 0, turn = 0;
     const LocalShape* shapes = local_shapes(c->words, n_shapes);
     Launch L;
-    CK(cudaEventRecord(c->fork_ev, c->stream));
     for (uint32_t cls = 0; cls < 8 + pa.n_shapes; ++cls, L.at += L.n) {
         L.n = 0;
         for (uint32_t b = 0; b < PLAN_SUB; ++b) L.n += w.bins[cls * PLAN_SUB + b];
@@ -268,12 +264,9 @@ int launch_classes(cfg_ctx* c, const RunWords& w, uint32_t& sides) {
         const LocalShape* sh = cls < 8 ? nullptr : &shapes[n_shapes - 1 - (cls - 8)];
         L.per = sh ? sh->slots : pa.per_cl;
         L.threads = sh ? sh->threads : 0;
-        const uint32_t q = turn++ % (cfg_ctx::SIDES + 1);   // 0: the context's own stream
-        if (q && !(sides >> q & 1)) {
-            CK(cudaStreamWaitEvent(c->side[q - 1], c->fork_ev, 0));
-            sides |= 1u << q;
-        }
-        const int rc = launch_one(c, L, q ? c->side[q - 1] : c->stream);
+        cudaStream_t s = nullptr;
+        CK(c->sides.on(c->stream, turn++, s));
+        const int rc = launch_one(c, L, s);
         if (rc) return rc;
     }
     return CFG_OK;
@@ -286,15 +279,10 @@ int launch_classes(cfg_ctx* c, const RunWords& w, uint32_t& sides) {
 int launch_planned(cfg_ctx* c, const RunWords& w) {
     int rc = ensure_arena(c, w.arena_slots);
     if (rc) return rc;
-    uint32_t sides = 0;   // bit q: side stream q - 1 has work
-    rc = launch_classes(c, w, sides);
-    for (uint32_t q = 1; q <= cfg_ctx::SIDES; ++q) {
-        if (!(sides >> q & 1)) continue;
-        if (rc) { cudaStreamSynchronize(c->side[q - 1]); continue; }   // a failed launch: nothing may outlive the call
-        CK(cudaEventRecord(c->join_ev[q - 1], c->side[q - 1]));
-        CK(cudaStreamWaitEvent(c->stream, c->join_ev[q - 1], 0));
-    }
-    return rc;
+    CK(c->sides.fork(c->stream));
+    rc = launch_classes(c, w);
+    const cudaError_t e = c->sides.join(c->stream, rc != CFG_OK);
+    return rc ? rc : e != cudaSuccess ? cuda_fail(c, e, "joining the table classes") : CFG_OK;
 }
 
 // The subgraphs in `work` again, with tables for want[i] slots.
@@ -490,10 +478,7 @@ int cfg_create(int device, const cfg_params* params, cfg_ctx** out) {
     if (cudaEventCreateWithFlags(&c->idle_ev, cudaEventDisableTiming) != cudaSuccess) { cfg_destroy(c); return CFG_ERR_CUDA; }
     for (auto& e : c->text_ev)
         if (cudaEventCreate(&e) != cudaSuccess) { cfg_destroy(c); return CFG_ERR_CUDA; }
-    if (cudaEventCreateWithFlags(&c->fork_ev, cudaEventDisableTiming) != cudaSuccess) { cfg_destroy(c); return CFG_ERR_CUDA; }
-    for (int q = 0; q < cfg_ctx::SIDES; ++q)
-        if (cudaStreamCreateWithFlags(&c->side[q], cudaStreamNonBlocking) != cudaSuccess ||
-            cudaEventCreateWithFlags(&c->join_ev[q], cudaEventDisableTiming) != cudaSuccess) { cfg_destroy(c); return CFG_ERR_CUDA; }
+    if (c->sides.create() != cudaSuccess) { cfg_destroy(c); return CFG_ERR_CUDA; }
     *out = c;
     return CFG_OK;
 }
@@ -818,7 +803,7 @@ void cfg_destroy(cfg_ctx* c) {
     cudaSetDevice(c->device);
     if (c->stream) cudaStreamSynchronize(c->stream);
     if (c->copy_stream) cudaStreamSynchronize(c->copy_stream);
-    for (auto& x : c->side) if (x) cudaStreamSynchronize(x);
+    c->sides.destroy();
     c->parse.release();
     c->ub.release();
     c->h_unitigs.release();
@@ -832,9 +817,6 @@ void cfg_destroy(cfg_ctx* c) {
     for (auto& e : c->piece_ev) if (e) cudaEventDestroy(e);
     if (c->idle_ev) cudaEventDestroy(c->idle_ev);
     for (auto& e : c->text_ev) if (e) cudaEventDestroy(e);
-    if (c->fork_ev) cudaEventDestroy(c->fork_ev);
-    for (auto& e : c->join_ev) if (e) cudaEventDestroy(e);
-    for (auto& x : c->side) if (x) cudaStreamDestroy(x);
     if (c->copy_stream) cudaStreamDestroy(c->copy_stream);
     if (c->stream) cudaStreamDestroy(c->stream);
     delete c;
