@@ -234,7 +234,6 @@ struct cfg_batch {
 
     // device collation of all jobs' lm-tigs (cfg_batch_unitigs)
     UnitigBuffers ub;
-    uint64_t ub_lmtigs = 0;             // lm-tigs the collation buffers hold
     DevBuf u_n, u_base, u_out, u_cur, u_err, u_cyc_work, u_cyc_scratch, u_cyc_out;
     std::vector<unsigned long long> h_out_base, h_ucur;
     std::vector<std::string> u_host;    // per job: unitigs joined on the host (cycles; redone jobs)
@@ -840,7 +839,7 @@ int cfg_batch_unitigs(cfg_batch* b, float* device_ms) {
     // buffers that already hold every lm-tig need no look at it (cudaMemGetInfo takes 0 to 80 ms
     // on a host that other processes' GPU calls share)
     unsigned long long cap = n_all;
-    if (n_all > b->ub_lmtigs) {
+    if (n_all > b->ub.held) {
         size_t fr = 0, tot = 0;
         BCK(cudaMemGetInfo(&fr, &tot));
         const unsigned long long per_lmtig = 240;   // bytes of collation buffers per lm-tig
@@ -858,8 +857,7 @@ int cfg_batch_unitigs(cfg_batch* b, float* device_ms) {
         uint32_t j1 = j0;
         unsigned long long n = 0;
         while (j1 < J && (j1 == j0 || n + jn[j1] <= cap)) { jb[j1] = n; n += jn[j1]; ++j1; }
-        if (!b->ub.ensure(n)) { b->ub_lmtigs = 0; return bfail(b, CFG_ERR_OOM, "collation buffers"); }
-        b->ub_lmtigs = std::max<uint64_t>(b->ub_lmtigs, n);
+        if (!b->ub.ensure(n, b->p.k)) return bfail(b, CFG_ERR_OOM, "collation buffers");
         BCK(cudaMemcpyAsync(b->u_base.as<unsigned long long>() + j0, jb.data() + j0, 8ull * (j1 - j0), cudaMemcpyHostToDevice,
                             b->stream));
         BCK(cudaEventRecord(b->ev[0], b->stream));

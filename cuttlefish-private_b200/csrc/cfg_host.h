@@ -130,7 +130,8 @@ struct UnitigBuffers {
     DevBuf b_label, b_tab, b_partner, b_X0, b_X1, b_fin, b_off, b_words, b_out, b_job, b_flip, b_sx, b_sw, b_len, b_ends;
     HostBuf h_words;              // page-locked copy of the collation's result words
     ulonglong2* ends = nullptr;   // both ends of each gathered lm-tig, packed for the pairing pass
-    uint32_t end_words = 2;       // 64-bit words per end there: 2 for k <= 63, 4 beyond (set from k)
+    uint32_t end_words = 2;       // 64-bit words per end there: 2 for k <= 63, 4 beyond
+    uint64_t held = 0;            // lm-tigs (of k-mers with end_words) that every buffer has room for
     uint32_t* len = nullptr;   // each gathered lm-tig's label length (the kernels after the gather read 4 bytes, not a record)
     uint8_t* flipb = nullptr;  // per lm-tig heading its chain's walked list: flip it
     uint32_t* job = nullptr;   // batch: each gathered lm-tig's job
@@ -145,7 +146,38 @@ struct UnitigBuffers {
     unsigned long long* out_off = nullptr;
     unsigned long long* words = nullptr;
     char* out = nullptr;
-    bool ensure(uint64_t n);
+    static constexpr uint32_t MAX_ROUNDS = 34;             // of the ranking: a count of active entries each
+    static constexpr size_t SLOT_BYTES = 8, RANK_BYTES = 16;   // a slot of the vertex table, a ranking record
+    // Room for n lm-tigs of k-mers of length k, in buffers that only grow.
+    bool ensure(uint64_t n, uint32_t k) {
+        // vertex table: 4 slots per lm-tig (at most half full: 2 ends per lm-tig); after
+        // pairing it holds the splitters' second ranking buffer (up to 2n records)
+        const uint64_t t = 4 * n + 64;
+        const uint64_t n2 = 2 * n + 2;
+        const uint32_t ew = k > 63 ? 4 : 2;
+        if (ew != end_words) held = 0;
+        end_words = ew;
+        if (!b_label.ensure(8 * (n + 1)) || !b_tab.ensure(SLOT_BYTES * t) ||
+            !b_partner.ensure(4 * n2) || !b_X0.ensure(RANK_BYTES * n2) || !b_X1.ensure(RANK_BYTES * n2) ||
+            !b_fin.ensure(4 * (n + 1)) || !b_sx.ensure(4 * n2) || !b_sw.ensure(4 * n2) ||
+            !b_off.ensure(8 * n2) || !b_words.ensure(8 * (8 + MAX_ROUNDS)) || !h_words.ensure(64) || !b_job.ensure(4 * (n + 1)) ||
+            !b_flip.ensure(n + 1) || !b_len.ensure(4 * (n + 1)) || !b_ends.ensure(16ull * end_words * (n + 1))) {
+            held = 0;   // a buffer that had to grow is gone
+            return false;
+        }
+        if (n > held) held = n;
+        len = b_len.as<uint32_t>();
+        ends = b_ends.as<ulonglong2>();
+        job = b_job.as<uint32_t>();
+        flipb = b_flip.as<uint8_t>();
+        label = (const char**)b_label.p; tab = b_tab.p; tab_n = t;
+        partner = b_partner.as<uint32_t>(); X[0] = b_X0.p; X[1] = b_X1.p;
+        fin = b_fin.as<uint32_t>(); out_off = b_off.as<unsigned long long>();
+        sx = b_sx.as<uint32_t>();
+        sw = b_sw.as<uint32_t>();
+        words = b_words.as<unsigned long long>();
+        return true;
+    }
     bool ensure_out(uint64_t bytes) {
         if (!b_out.ensure(bytes)) return false;
         out = b_out.as<char>();
@@ -156,6 +188,7 @@ struct UnitigBuffers {
                          &b_flip, &b_sx, &b_sw, &b_len, &b_ends};
         for (DevBuf* b : all) b->release();
         h_words.release();
+        held = 0;
     }
 };
 // ... and what it produced: `bytes` of FASTA records at out, the unitigs among them,

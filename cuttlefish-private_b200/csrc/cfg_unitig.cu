@@ -46,6 +46,8 @@ using EndSlot = uint2;
 // once resolved), the farthest known ancestor (the head once resolved), and the label
 // bases of the entries between them.
 struct RankRec { uint32_t P, R; unsigned long long A; };
+static_assert(sizeof(EndSlot) == UnitigBuffers::SLOT_BYTES && sizeof(RankRec) == UnitigBuffers::RANK_BYTES,
+              "UnitigBuffers sizes the buffers");
 
 // Ranking marks: an entry that no splitter's walk passed lies on a closed chain.
 constexpr uint32_t UNOWNED = 0xfffffffeu;
@@ -313,7 +315,7 @@ __device__ __forceinline__ bool failed(const uint32_t* err) { return *err & (DER
 // act[r] counts the entries still unresolved after round r, and a round does nothing once
 // none is, or once a round resolved none (what is left lies on closed chains; an open chain
 // resolves some entries in every round).
-constexpr uint32_t MAX_ROUNDS = 34;
+constexpr uint32_t MAX_ROUNDS = UnitigBuffers::MAX_ROUNDS;
 __device__ __forceinline__ bool round_runs(const unsigned long long* act, uint32_t r) {
     return r == 0 || (act[r - 1] && !(r > 1 && act[r - 1] == act[r - 2]));
 }
@@ -766,30 +768,6 @@ __global__ void __launch_bounds__(256) k_cy_rotate(const uint32_t* __restrict__ 
 
 }  // namespace
 
-bool UnitigBuffers::ensure(uint64_t n) {
-    // vertex table: 4 slots per lm-tig (at most half full: 2 ends per lm-tig); after
-    // pairing it holds the splitters' second ranking buffer (up to 2n records)
-    const uint64_t t = 4 * n + 64;
-    const uint64_t n2 = 2 * n + 2;
-    if (!b_label.ensure(8 * (n + 1)) || !b_tab.ensure(sizeof(EndSlot) * t) ||
-        !b_partner.ensure(4 * n2) || !b_X0.ensure(sizeof(RankRec) * n2) || !b_X1.ensure(sizeof(RankRec) * n2) ||
-        !b_fin.ensure(4 * (n + 1)) || !b_sx.ensure(4 * n2) || !b_sw.ensure(4 * n2) ||
-        !b_off.ensure(8 * n2) || !b_words.ensure(8 * (8 + MAX_ROUNDS)) || !h_words.ensure(64) || !b_job.ensure(4 * (n + 1)) || !b_flip.ensure(n + 1) ||
-        !b_len.ensure(4 * (n + 1)) || !b_ends.ensure(16ull * end_words * (n + 1)))
-        return false;
-    len = b_len.as<uint32_t>();
-    ends = b_ends.as<ulonglong2>();
-    job = b_job.as<uint32_t>();
-    flipb = b_flip.as<uint8_t>();
-    label = (const char**)b_label.p; tab = b_tab.p; tab_n = t;
-    partner = b_partner.as<uint32_t>(); X[0] = b_X0.p; X[1] = b_X1.p;
-    fin = b_fin.as<uint32_t>(); out_off = b_off.as<unsigned long long>();
-    sx = b_sx.as<uint32_t>();
-    sw = b_sw.as<uint32_t>();
-    words = b_words.as<unsigned long long>();
-    return true;
-}
-
 int collate_cycles_on_device(UnitigBuffers& ub, uint64_t n, uint64_t m, uint32_t k, uint32_t* err, DevBuf& work,
                              DevBuf& scratch, DevBuf& out, cudaStream_t s, uint64_t& out_bytes, uint64_t& n_cycles,
                              const uint32_t* job, std::vector<CycleRecord>* records) {
@@ -866,8 +844,7 @@ int collate_cycles_on_device(UnitigBuffers& ub, uint64_t n, uint64_t m, uint32_t
 int collate_device(const UnitigInput& in, UnitigBuffers& ub, cudaStream_t s, UnitigResult& res) {
     res = UnitigResult{};
     const uint64_t n = in.n;
-    ub.end_words = in.k > 63 ? 4 : 2;
-    if (!ub.ensure(n)) return CFG_ERR_OOM;
+    if (!ub.ensure(n, in.k)) return CFG_ERR_OOM;
     if (cudaMemsetAsync(ub.words, 0, sizeof(unsigned long long) * (8 + MAX_ROUNDS), s) != cudaSuccess) return CFG_ERR_CUDA;
     // [0] output bytes, [1] unitigs, [2] cycle lm-tigs, [3] the error word, [4] splitters,
     // [5] insert tiles taken, [6] splitters taken by walks, [8..] active entries after each round

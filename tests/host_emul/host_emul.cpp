@@ -1,6 +1,7 @@
-// host_emul.cpp -- host helpers of the library (csrc/cfg_sides.h) on a
+// host_emul.cpp -- host helpers of the library (csrc/cfg_sides.h, cfg_host.h) on a
 // stand-in CUDA runtime that records every call and fails the one it is told to, for the
 // tests: no GPU is involved, and no call fails on a real one.
+#include "cfg_host.h"
 #include "cfg_sides.h"
 
 #include <cstdint>
@@ -14,6 +15,9 @@ struct Op { Kind kind; const void* stream; const void* event; };
 std::vector<Op> g_ops;
 long g_calls = 0, g_fail_at = -1;   // calls that may fail so far; the one that does
 uintptr_t g_next = 0x1000;
+
+size_t g_room = SIZE_MAX, g_asked = 0;   // device bytes left to give out; bytes given out since the last reset
+std::map<const void*, size_t> g_blocks;
 
 cudaError_t step() { return g_calls++ == g_fail_at ? cudaErrorUnknown : cudaSuccess; }
 
@@ -44,6 +48,39 @@ cudaError_t cudaStreamWaitEvent(cudaStream_t s, cudaEvent_t ev, unsigned) {
     return e;
 }
 cudaError_t cudaStreamSynchronize(cudaStream_t s) { g_ops.push_back(Op{SYNC, s, nullptr}); return cudaSuccess; }
+
+cudaError_t cudaMalloc(void** p, size_t n) {
+    if (n > g_room) return cudaErrorMemoryAllocation;
+    g_room -= n; g_asked += n;
+    *p = (void*)(g_next += 256);   // never looked into
+    g_blocks[*p] = n;
+    return cudaSuccess;
+}
+cudaError_t cudaFree(void* p) {
+    g_room += g_blocks[p];
+    g_blocks.erase(p);
+    return cudaSuccess;
+}
+cudaError_t cudaMallocHost(void** p, size_t) { *p = (void*)(g_next += 256); return cudaSuccess; }
+cudaError_t cudaFreeHost(void*) { return cudaSuccess; }
+cudaError_t cudaGetLastError() { return cudaSuccess; }
+
+// Collation buffers for n lm-tigs of k-mers of length k, twice with the device full after
+// the first, then for `more` lm-tigs there is no room for.  -> 0, or the promise broken.
+int unitig_buffers(uint64_t n, uint64_t more, uint32_t k) {
+    cfg::UnitigBuffers ub;
+    g_room = SIZE_MAX;
+    if (!ub.ensure(n, k) || ub.held != n) return 1;
+    g_room = 0;
+    g_asked = 0;
+    if (!ub.ensure(n, k) || g_asked) return 2;       // what is held is enough
+    if (ub.held != n) return 3;
+    if (ub.ensure(more, k) || ub.held != 0) return 4;   // a failed call lost a buffer, and says so
+    g_room = SIZE_MAX;
+    if (!ub.ensure(n, k) || ub.held != n) return 5;
+    ub.release();
+    return ub.held != 0 ? 6 : 0;
+}
 
 // One pass of `launches` launches in which call number fail_at fails (-1: none; the calls
 // of create() are not counted).  -> 0: the pass kept its promise, else which one it broke;
