@@ -55,11 +55,10 @@ struct HostBuf {
 // Device buffers of the text parser (cfg_parse.cu): per-chunk scan words, break
 // ranks, the fragment table and the packed stream it produces.
 struct ParseBuffers {
-    DevBuf cf, cb, ck, br, fo, pn, pbb, foff, flen, tot, pk, tf, tp, tm, cpf, cps;
+    DevBuf cf, cb, ck, br, fo, pn, pbb, foff, flen, tot, pk, gw, sp, cpf, cps;
     uint32_t* chunk_f = nullptr;
-    uint16_t* thread_f = nullptr;   // per group of every chunk: the chunk's function before its bytes
-    uint32_t* thread_pre = nullptr; // per group of every chunk: the chunk's bases and breaks before its bytes
-    uint32_t* thread_m = nullptr;   // per group of every chunk: which of its bytes are bases, and breaks
+    uint32_t* group_w = nullptr;    // per group of every chunk: the chunk's function before its bytes, then its emissions
+    uint32_t* step_pre = nullptr;   // per 32 groups: the chunk's bases and breaks before them
     uint32_t* chunk_part_f = nullptr;             // per 1024 chunks: transfer function,
     unsigned long long* chunk_part_s = nullptr;   // bases and breaks
     unsigned long long *chunk_b = nullptr, *chunk_k = nullptr, *brk_rank = nullptr, *frag_out = nullptr;
@@ -70,13 +69,12 @@ struct ParseBuffers {
     uint64_t* packed = nullptr;
     uint64_t n_frags = 0, n_bases = 0;
     bool ensure_chunks(uint64_t n) {
-        if (!cf.ensure(4 * n) || !cb.ensure(8 * n) || !ck.ensure(8 * n) || !tf.ensure(2 * 256 * n) || !tp.ensure(4 * 256 * n) ||
-            !tm.ensure(4 * 256 * n) || !cpf.ensure(4 * (n / 1024 + 1)) || !cps.ensure(16 * (n / 1024 + 1)))
+        if (!cf.ensure(4 * n) || !cb.ensure(8 * n) || !ck.ensure(8 * n) || !gw.ensure(4 * 256 * n) || !sp.ensure(4 * 8 * n) ||
+            !cpf.ensure(4 * (n / 1024 + 1)) || !cps.ensure(16 * (n / 1024 + 1)))
             return false;
         chunk_f = cf.as<uint32_t>(); chunk_b = cb.as<unsigned long long>(); chunk_k = ck.as<unsigned long long>();
-        thread_f = tf.as<uint16_t>();
-        thread_pre = tp.as<uint32_t>();
-        thread_m = tm.as<uint32_t>();
+        group_w = gw.as<uint32_t>();
+        step_pre = sp.as<uint32_t>();
         chunk_part_f = cpf.as<uint32_t>(); chunk_part_s = cps.as<unsigned long long>();
         return true;
     }
@@ -96,7 +94,7 @@ struct ParseBuffers {
         return true;
     }
     void release() {
-        DevBuf* all[] = {&cf, &cb, &ck, &br, &fo, &pn, &pbb, &foff, &flen, &tot, &pk, &tf, &tp, &tm, &cpf, &cps};
+        DevBuf* all[] = {&cf, &cb, &ck, &br, &fo, &pn, &pbb, &foff, &flen, &tot, &pk, &gw, &sp, &cpf, &cps};
         for (DevBuf* b : all) b->release();
     }
 };

@@ -14,16 +14,21 @@
 // (a scan), so every chunk runs independently:
 //   A  transfer function of every chunk (and of every group's bytes before it, kept
 //      for C)                                       B  scan: each chunk's start state
-//   C  each group's emissions as two 16-bit masks (kept for E and G), the chunk's bases
-//      and breaks (and those before every group)    D  scan: each chunk's offsets
+//   C  each group's emissions as two 16-bit masks (kept for E and G, in the word that held
+//      A's function), bases and breaks of the chunk and before every 32 of its groups
+//                                                   D  scan: each chunk's offsets
 //   E  the base rank of every break                F  fragments: lengths, keep, offsets
 //   G  bases written 2 bits each into the packed stream.
 // A and C give a warp a whole chunk, 32 groups of 16 bytes at a time: no barrier, every
 // load of the chunk in flight at once, the scan carried in registers.  E and G visit only
-// the groups with breaks, or bases, to place; what is done with a group's 16 bytes is in
-// cfg_parse_thread.cuh.  Bound: instruction issue (the text is read three times, 0.3 ms of
-// the 1.75 ms that 640 MB of FASTQ take; 8.8 ms with a byte-by-byte walk of the groups that
-// hold a newline, CTA-wide scans and one-CTA scans over the chunks).
+// the groups with breaks, or bases, to place, and find what is before a group by a scan over
+// the warp: 4 bytes per group and 4 per 32 groups are all that is kept, 0.26 bytes per byte of
+// text (a prefix and the masks of every group, in words of their own beside A's function: 0.63
+// bytes, and 1.74 ms where this takes 1.63; with one group to a lane the scans made it 1.81).
+// What is done with a group's 16 bytes is in cfg_parse_thread.cuh.  Bound: instruction issue
+// (the text is read three times, 0.3 ms of the 1.63 ms that 630 MB of FASTQ take; 8.8 ms with a
+// byte-by-byte walk of the groups that hold a newline, CTA-wide scans and one-CTA scans over
+// the chunks).
 #include "cuttlefish_gpu.h"
 #include "cfg_host.h"
 #include "cfg_internal.h"
@@ -42,9 +47,9 @@ struct ParseArgs {
     uint64_t bytes, n_chunks;
     FsmBits fsm;
     uint32_t* chunk_f;             // A: transfer function; B: start state
-    uint16_t* thread_f;            // A: per group, the chunk's function before it
-    uint32_t* thread_pre;          // C: per group, the chunk's bases and breaks before it
-    uint32_t* thread_m;            // C: per group, its bytes that are bases (low half) and breaks (high half)
+    uint32_t* group_w;             // A: per group, the chunk's function before it; C: its bytes that are bases (low
+                                   // half) and breaks (high half)
+    uint32_t* step_pre;            // C: per 32 groups, the chunk's bases and breaks before them
     uint32_t* part_f;              // B: transfer function of every 1024 chunks
     unsigned long long* part_s;    // C: bases and breaks of every 1024 chunks
     unsigned long long* chunk_b;   // C: bases; D: bases before the chunk
@@ -106,7 +111,7 @@ __global__ void __launch_bounds__(TPB) k_parse_transfer(ParseArgs a) {
             const uint32_t t = i * 32 + lane;
             const Fn x = warp_scan_fn(thread_fn(a.fsm, g[i], bytes_at(a, c * CHUNK + (uint64_t)t * BPT)), lane);
             const Fn up{__shfl_up_sync(FULL, x.lo, 1), __shfl_up_sync(FULL, x.hi, 1)};
-            a.thread_f[c * TPB + t] = (uint16_t)fn_bits(lane ? fn_then(carry, up) : carry);
+            a.group_w[c * TPB + t] = fn_bits(lane ? fn_then(carry, up) : carry);
             carry = fn_then(carry, shfl_fn(x, 31));
         }
         if (lane == 0) a.chunk_f[c] = fn_bits(carry);
@@ -182,7 +187,7 @@ __global__ void __launch_bounds__(TPB) k_parse_counts(ParseArgs a) {
 #pragma unroll
         for (uint32_t i = 0; i < WARP_GROUPS; ++i) {
             g[i] = load_group(a, c * CHUNK + (uint64_t)(i * 32 + lane) * BPT);
-            tf[i] = a.thread_f[c * TPB + i * 32 + lane];
+            tf[i] = a.group_w[c * TPB + i * 32 + lane];
         }
         const uint32_t st = a.chunk_f[c];
         uint32_t carry = 0;   // bases | breaks << 16 before this step's groups (a chunk holds 4096 bytes)
@@ -190,16 +195,9 @@ __global__ void __launch_bounds__(TPB) k_parse_counts(ParseArgs a) {
         for (uint32_t i = 0; i < WARP_GROUPS; ++i) {
             const uint32_t t = i * 32 + lane;
             const Emits e = thread_emits(a.fsm, f_at(tf[i], st), g[i], bytes_at(a, c * CHUNK + (uint64_t)t * BPT));
-            const uint32_t own = pre_pack(popc32(e.base), popc32(e.brk));
-            uint32_t x = own;
-#pragma unroll
-            for (int d = 1; d < 32; d <<= 1) {
-                const uint32_t y = __shfl_up_sync(FULL, x, d);
-                if (lane >= (uint32_t)d) x += y;
-            }
-            a.thread_pre[c * TPB + t] = carry + x - own;
-            a.thread_m[c * TPB + t] = e.base | (e.brk << 16);
-            carry += __shfl_sync(FULL, x, 31);
+            if (lane == 0) a.step_pre[c * WARP_GROUPS + i] = carry;
+            a.group_w[c * TPB + t] = emits_word(e);
+            carry += __reduce_add_sync(FULL, emits_counts(e));
         }
         if (lane == 0) {
             a.chunk_b[c] = pre_bases(carry); a.chunk_k[c] = pre_breaks(carry);
@@ -263,17 +261,40 @@ __global__ void __launch_bounds__(TPB) k_parse_offsets(ParseArgs a) {
     }
 }
 
-__device__ __forceinline__ Emits group_emits(uint32_t m) { return Emits{m & 0xFFFFu, m >> 16}; }
+// Bases and breaks of the chunk before the lane's groups: the warp's lanes hold `own` each, in
+// order, and its first group starts step `step`.
+__device__ __forceinline__ uint32_t groups_pre(const ParseArgs& a, uint64_t step, uint32_t own) {
+    const uint32_t lane = threadIdx.x & 31;
+    uint32_t x = own;
+#pragma unroll
+    for (int d = 1; d < 32; d <<= 1) {
+        const uint32_t y = __shfl_up_sync(FULL, x, d);
+        if (lane >= (uint32_t)d) x += y;
+    }
+    return a.step_pre[step] + x - own;
+}
 
 // E: for every break, the number of bases before it; break NB (after the text) closes
-// the last fragment.  Only groups that emit a break are looked at.
+// the last fragment.  Four groups to a lane, so that the warp's scan serves 128 of them;
+// a warp runs whole, and within one chunk.
 __global__ void __launch_bounds__(TPB) k_parse_breaks(ParseArgs a) {
-    const uint64_t n = a.n_chunks * TPB, stride = (uint64_t)gridDim.x * TPB;
+    constexpr uint32_t N = 4;
+    const uint64_t n = a.n_chunks * (TPB / N), stride = (uint64_t)gridDim.x * TPB;
     for (uint64_t i = (uint64_t)blockIdx.x * TPB + threadIdx.x; i < n; i += stride) {
-        const Emits e = group_emits(a.thread_m[i]);
-        if (!e.brk) continue;
-        const uint32_t pre = a.thread_pre[i];
-        emit_breaks(e, a.chunk_b[i / TPB] + pre_bases(pre), a.chunk_k[i / TPB] + pre_breaks(pre), a.brk_rank);
+        const uint4 m = ((const uint4*)a.group_w)[i];
+        if (!__any_sync(FULL, (m.x | m.y | m.z | m.w) >> 16)) continue;
+        const uint32_t w[N] = {m.x, m.y, m.z, m.w};
+        uint32_t own = 0;
+#pragma unroll
+        for (uint32_t j = 0; j < N; ++j) own += emits_counts(word_emits(w[j]));
+        uint32_t pre = groups_pre(a, (i / 32) * N, own);
+        const unsigned long long r = a.chunk_b[i / (TPB / N)], kk = a.chunk_k[i / (TPB / N)];
+#pragma unroll
+        for (uint32_t j = 0; j < N; ++j) {
+            const Emits e = word_emits(w[j]);
+            emit_breaks(e, r + pre_bases(pre), kk + pre_breaks(pre), a.brk_rank);
+            pre += emits_counts(e);
+        }
     }
     if (blockIdx.x == 0 && threadIdx.x == 0) a.brk_rank[a.chunk_k[a.n_chunks]] = a.chunk_b[a.n_chunks];
 }
@@ -387,16 +408,25 @@ struct AtomicOr64 {
     }
 };
 
-// G: every kept base to its place in the packed stream (MSB-first, 32 per word).  Only
-// groups that emit a base read their bytes.
+// G: every kept base to its place in the packed stream (MSB-first, 32 per word).  Two
+// groups to a lane (as in E); only groups that emit a base read their bytes.
 __global__ void __launch_bounds__(TPB) k_parse_pack(ParseArgs a) {
-    const uint64_t n = a.n_chunks * TPB, stride = (uint64_t)gridDim.x * TPB;
+    constexpr uint32_t N = 2;
+    const uint64_t n = a.n_chunks * (TPB / N), stride = (uint64_t)gridDim.x * TPB;
     for (uint64_t i = (uint64_t)blockIdx.x * TPB + threadIdx.x; i < n; i += stride) {
-        const Emits e = group_emits(a.thread_m[i]);
-        if (!e.base) continue;
-        const uint32_t pre = a.thread_pre[i];
-        emit_pack(e, load_group(a, i * BPT), a.chunk_b[i / TPB] + pre_bases(pre), a.chunk_k[i / TPB] + pre_breaks(pre),
-                  a.frag_out, a.brk_rank, a.packed, AtomicOr64{});
+        const uint2 m = ((const uint2*)a.group_w)[i];
+        if (!__any_sync(FULL, (m.x | m.y) & 0xFFFFu)) continue;
+        const uint32_t w[N] = {m.x, m.y};
+        uint32_t pre = groups_pre(a, (i / 32) * N, emits_counts(word_emits(m.x)) + emits_counts(word_emits(m.y)));
+        const unsigned long long r = a.chunk_b[i / (TPB / N)], kk = a.chunk_k[i / (TPB / N)];
+#pragma unroll
+        for (uint32_t j = 0; j < N; ++j) {
+            const Emits e = word_emits(w[j]);
+            if (e.base)
+                emit_pack(e, load_group(a, (i * N + j) * BPT), r + pre_bases(pre), kk + pre_breaks(pre), a.frag_out,
+                          a.brk_rank, a.packed, AtomicOr64{});
+            pre += emits_counts(e);
+        }
     }
 }
 
@@ -409,10 +439,10 @@ int parse_text_device(const uint8_t* d_text, uint64_t bytes, int fastq, uint32_t
     a.fsm = pack_fsm(fastq ? fastq_fsm() : fasta_fsm());
     const uint64_t nc = a.n_chunks;
     if (!pb.ensure_chunks(nc + 1)) return CFG_ERR_OOM;
-    a.chunk_f = pb.chunk_f; a.chunk_b = pb.chunk_b; a.chunk_k = pb.chunk_k; a.thread_f = pb.thread_f;
-    a.thread_pre = pb.thread_pre; a.thread_m = pb.thread_m; a.part_f = pb.chunk_part_f; a.part_s = pb.chunk_part_s;
+    a.chunk_f = pb.chunk_f; a.chunk_b = pb.chunk_b; a.chunk_k = pb.chunk_k;
+    a.group_w = pb.group_w; a.step_pre = pb.step_pre; a.part_f = pb.chunk_part_f; a.part_s = pb.chunk_part_s;
     const unsigned wgrid = (unsigned)std::min<uint64_t>((nc + TPB / 32 - 1) / (TPB / 32), 148ull * 32);   // a warp per chunk
-    const unsigned grid = (unsigned)std::min<uint64_t>(std::max<uint64_t>(nc, 1), 148ull * 32);           // a thread per group
+    const unsigned bgrid = (unsigned)std::min<uint64_t>((nc + 3) / 4, 148ull * 32), pgrid = (unsigned)std::min<uint64_t>((nc + 1) / 2, 148ull * 32);
     const unsigned sgrid = (unsigned)std::max<uint64_t>((nc + SCAN_CHUNKS - 1) / SCAN_CHUNKS, 1);
     if (cudaMemsetAsync(a.part_s, 0, 16ull * sgrid, s) != cudaSuccess) return CFG_ERR_CUDA;
     if (nc) {
@@ -430,7 +460,7 @@ int parse_text_device(const uint8_t* d_text, uint64_t bytes, int fastq, uint32_t
     const uint64_t n_frag = tot[1] + 1;
     if (!pb.ensure_frags(n_frag)) return CFG_ERR_OOM;
     a.brk_rank = pb.brk_rank;
-    if (nc) k_parse_breaks<<<grid, TPB, 0, s>>>(a);
+    if (nc) k_parse_breaks<<<bgrid, TPB, 0, s>>>(a);
     else if (cudaMemsetAsync(a.brk_rank, 0, 8, s) != cudaSuccess) return CFG_ERR_CUDA;
     FragArgs f{};
     f.brk_rank = pb.brk_rank; f.n_frag = n_frag; f.k = k; f.out = pb.frag_out;
@@ -449,7 +479,7 @@ int parse_text_device(const uint8_t* d_text, uint64_t bytes, int fastq, uint32_t
     if (!pb.ensure_packed(words + 4)) return CFG_ERR_OOM;
     if (cudaMemsetAsync(pb.packed, 0, 8 * (words + 4), s) != cudaSuccess) return CFG_ERR_CUDA;
     a.packed = pb.packed; a.frag_out = pb.frag_out;
-    if (nc) k_parse_pack<<<grid, TPB, 0, s>>>(a);
+    if (nc) k_parse_pack<<<pgrid, TPB, 0, s>>>(a);
     if (cudaGetLastError() != cudaSuccess) return CFG_ERR_CUDA;
     return CFG_OK;
 }

@@ -202,6 +202,11 @@ CFG_PHD Fn thread_fn(const FsmBits& f, const Group& g, uint32_t nb) {
 }
 CFG_PHD uint32_t thread_transfer(const FsmBits& f, const Group& g, uint32_t nb) { return fn_bits(thread_fn(f, g, nb)); }
 
+// Bases (low 16 bits) and breaks (high 16 bits) within one chunk, of at most 4096 bytes.
+CFG_PHD uint32_t pre_pack(uint32_t eb, uint32_t ek) { return eb | (ek << 16); }
+CFG_PHD uint32_t pre_bases(uint32_t p) { return p & 0xFFFFu; }
+CFG_PHD uint32_t pre_breaks(uint32_t p) { return p >> 16; }
+
 // What the group's nbytes bytes emit from state st: bit i of base (brk) -- byte i is a base
 // (a break).
 struct Emits { uint32_t base, brk; };
@@ -229,6 +234,12 @@ CFG_PHD Emits thread_emits(const FsmBits& f, uint32_t st, const Group& g, uint32
     const uint32_t a = acgt_mask(g);
     return Emits{a & seq, brk | (seq & ~a)};
 }
+
+// A group's emissions as one word: what pass C leaves for E and G.
+CFG_PHD uint32_t emits_word(Emits e) { return e.base | (e.brk << 16); }
+CFG_PHD Emits word_emits(uint32_t m) { return Emits{m & 0xFFFFu, m >> 16}; }
+// Its bases and breaks.
+CFG_PHD uint32_t emits_counts(Emits e) { return pre_pack(popc32(e.base), popc32(e.brk)); }
 
 // Bases and breaks the group emits from state st.
 CFG_PHD void thread_counts(const FsmBits& f, uint32_t st, const Group& g, uint32_t nbytes, uint32_t& nb, uint32_t& nk) {
@@ -307,12 +318,6 @@ CFG_PHD void thread_pack(const FsmBits& f, uint32_t st, const Group& g, uint32_t
     (void)nk;
     if (nb) emit_pack(thread_emits(f, st, g, nbytes), g, r, kk, frag_out, brk_rank, packed, or64);
 }
-
-// A thread's exclusive prefix of bases (low 16 bits) and breaks (high 16 bits) within its
-// chunk; the 255 threads before it hold at most 4080 bytes.
-CFG_PHD uint32_t pre_pack(uint32_t eb, uint32_t ek) { return eb | (ek << 16); }
-CFG_PHD uint32_t pre_bases(uint32_t p) { return p & 0xFFFFu; }
-CFG_PHD uint32_t pre_breaks(uint32_t p) { return p >> 16; }
 
 // After pass D: bases and breaks before thread t's bytes (r, kk) and its own (nb, nk),
 // from pass C's per-thread prefixes (the next thread's, or the chunk's totals for the

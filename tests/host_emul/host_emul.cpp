@@ -82,6 +82,16 @@ int unitig_buffers(uint64_t n, uint64_t more, uint32_t k) {
     return ub.held != 0 ? 6 : 0;
 }
 
+// Device bytes that the text parser's per-chunk state of `bytes` bytes of text asks for.
+uint64_t parse_state_bytes(uint64_t bytes) {
+    cfg::ParseBuffers pb;
+    g_room = SIZE_MAX;
+    g_asked = 0;
+    const bool ok = pb.ensure_chunks((bytes + 4095) / 4096 + 1);
+    pb.release();
+    return ok ? g_asked : 0;
+}
+
 // One pass of `launches` launches in which call number fail_at fails (-1: none; the calls
 // of create() are not counted).  -> 0: the pass kept its promise, else which one it broke;
 // *calls: the calls that could have failed.
