@@ -1,13 +1,16 @@
 // cfg_parse_thread.cuh -- what one thread of the device text parser (cfg_parse.cu) does
 // with its 16 bytes, as __host__ __device__ code: the kernels run these steps on the
-// GPU, and a host harness in the tests runs the very same steps over every (chunk,
-// thread) of a text to check them on a CPU.
+// GPU, and host harnesses in the tests run them over every group of a text on a CPU.  The
+// steps are thread_fn, thread_emits, emits_word and its inverse, emit_breaks and emit_pack;
+// thread_transfer, thread_counts, thread_breaks, thread_pack and thread_span put them
+// together for the harness that checks one step at a time, and no kernel calls those.
 //
 // Bytes have five classes (newline, '>', a base letter, '\r', other); a finite-state
 // machine over the classes (the line structure of FASTA or FASTQ) gives each byte an
 // emission: skipped, a base, or a break (a non-ACGT character, a record boundary).
 //
-// A group is never walked byte by byte.  In both machines a run of base and other bytes
+// A group is never walked byte by byte.  In both machines (runs_alike, checked when they are
+// compiled) a run of base and other bytes
 // moves every state once (one class map, idempotent) and emits alike from its first byte to
 // its last -- bases and breaks from the states of a sequence line, nothing from the others
 // -- so only the delimiters ('\n', '\r', and '>' where it is one) step the state.  Word-wise
@@ -67,11 +70,11 @@ struct FsmBits {
     unsigned long long cf_lo;
     uint32_t cf_hi;
     uint32_t n, start;
-    // word-wise groups: loop_mask bit s -- state s stays s on a base and on an other byte;
-    // gt_other -- '>' has the next states and emissions of an other byte in every state
-    // (it is then no delimiter); bo_idem -- bases and other bytes have one class map, and
-    // it is idempotent (a group of them composes to that map); seq_mask bit s -- runs that
-    // start in state s emit (base: E_BASE, other: E_BREAK; from the other states E_SKIP)
+    // word-wise groups: gt_other -- '>' has the next states and emissions of an other byte in
+    // every state (it is then no delimiter); seq_mask bit s -- runs that start in state s emit
+    // (base: E_BASE, other: E_BREAK; from the other states E_SKIP).  Of the machine, read by no
+    // step: loop_mask bit s -- state s stays s on a base and on an other byte; bo_idem -- bases
+    // and other bytes have one class map, and it is idempotent
     uint32_t loop_mask, gt_other, bo_idem, seq_mask;
     Fn run, nl, cr, gt;   // the class maps of a run, '\n', '\r' and '>'
 };
@@ -349,6 +352,20 @@ struct Fsm {
     uint32_t n, start;
 };
 
+// What the word-wise steps take for granted: bases and other bytes have one class map, and it
+// is idempotent; a run of them emits its bases and breaks on its other bytes, or nothing, and
+// does the same from its second byte on as from its first.
+constexpr bool runs_alike(const Fsm& m) {
+    for (uint32_t st = 0; st < m.n; ++st) {
+        const uint32_t nx = m.next[st][C_BASE];
+        if (m.next[st][C_OTHER] != nx || m.next[nx][C_BASE] != nx) return false;
+        const bool seq = m.emit[st][C_BASE] == E_BASE;
+        if (m.emit[st][C_BASE] != (seq ? E_BASE : E_SKIP) || m.emit[st][C_OTHER] != (seq ? E_BREAK : E_SKIP)) return false;
+        if ((m.emit[nx][C_BASE] == E_BASE) != seq) return false;
+    }
+    return true;
+}
+
 inline FsmBits pack_fsm(const Fsm& m) {
     FsmBits b{};
     b.n = m.n; b.start = m.start;
@@ -363,8 +380,6 @@ inline FsmBits pack_fsm(const Fsm& m) {
         }
         if (c < 4) b.cf_lo |= (unsigned long long)F << (15 * c); else b.cf_hi = F;
     }
-    // word-wise groups (cfg_parse_thread.cuh): states that loop on bases and other bytes,
-    // '>' as an other byte, and one idempotent map for bases and other bytes
     b.gt_other = 1;
     b.bo_idem = 1;
     for (uint32_t st = 0; st < m.n; ++st) {
@@ -379,7 +394,7 @@ inline FsmBits pack_fsm(const Fsm& m) {
     return b;
 }
 
-inline Fsm fasta_fsm() {
+constexpr Fsm fasta_fsm() {
     // states: 0 line start before any record, 1 inside such a line, 2 header,
     // 3 line start inside a record, 4 sequence line
     Fsm m{};
@@ -397,7 +412,7 @@ inline Fsm fasta_fsm() {
     return m;
 }
 
-inline Fsm fastq_fsm() {
+constexpr Fsm fastq_fsm() {
     // states: 0 before a record (blank lines skipped), 1 header line, 2 sequence line,
     // 3 '+' line, 4 quality line
     Fsm m{};
@@ -413,6 +428,8 @@ inline Fsm fastq_fsm() {
     set(4, C_NL, 0, E_SKIP);
     return m;
 }
+
+static_assert(runs_alike(fasta_fsm()) && runs_alike(fastq_fsm()), "the word-wise steps read both machines' runs alike");
 
 }  // namespace parse
 }  // namespace cfg

@@ -97,4 +97,34 @@ int parse_emul(const uint8_t* text, uint64_t bytes, int fastq, uint32_t k, uint6
 
 void parse_emul_free(void* p) { std::free(p); }
 
+// runs_alike against the byte-by-byte meaning of it, on both machines with one table entry
+// changed to every other value: runs of two and three bases and other bytes must move every
+// state and emit as a run's first byte says.  -> entries it judged wrongly.
+int runs_alike_mismatches() {
+    int bad = 0;
+    for (const Fsm& m0 : {fasta_fsm(), fastq_fsm()}) {
+        for (uint32_t at = 0; at < m0.n * NCLASS * 2; ++at)
+            for (uint32_t v = 0; v < 5; ++v) {
+                Fsm m = m0;
+                const uint32_t s = at / 2 / NCLASS, c = at / 2 % NCLASS;
+                if (at & 1) { if (v > 2) continue; m.emit[s][c] = (uint8_t)v; } else m.next[s][c] = (uint8_t)v;
+                bool alike = true;
+                for (uint32_t st = 0; st < m.n; ++st)
+                    for (uint32_t run = 0; run < 8; ++run) {   // three bytes, bit set: an other byte
+                        const bool seq = m.emit[st][C_BASE] == E_BASE;
+                        const uint32_t to = m.next[st][C_BASE];
+                        uint32_t x = st;
+                        for (uint32_t i = 0; i < 3; ++i) {
+                            const uint32_t cl = run >> i & 1 ? C_OTHER : C_BASE;
+                            alike = alike && m.emit[x][cl] == (!seq ? E_SKIP : cl == C_BASE ? E_BASE : E_BREAK);
+                            x = m.next[x][cl];
+                            alike = alike && x == to;
+                        }
+                    }
+                bad += alike != runs_alike(m);
+            }
+    }
+    return bad;
+}
+
 }  // extern "C"

@@ -72,3 +72,8 @@ def test_parse_by_stored_words(route, case):
         host_parse.check(route, fastq_text(rng, 31, int(rng.integers(50, 3_000))), 31)
     else:
         host_parse.test_edge_texts(route) if case == 5 else host_parse.test_fasta_long_lines_and_crlf(route)
+
+
+def test_machines_are_held_to_what_the_word_steps_assume(route):
+    """The compile-time check of the parser's machines tells exactly those whose runs the word-wise steps read rightly."""
+    assert route.runs_alike_mismatches() == 0
