@@ -197,9 +197,6 @@ struct cfg_batch {
     int words = 1;
     cudaStream_t stream = nullptr;
     cudaEvent_t ev[2] = {};
-    static constexpr int SIDES = 3;     // capture only: the table classes' branches of the graph
-    cudaStream_t side[SIDES] = {};
-    cudaEvent_t fork_ev = nullptr, join_ev[SIDES] = {};
     std::string err;
     cfg_batch_tuning tune{4, 512, 100, 0, 0.f};
     uint32_t G_params = 16384;
@@ -331,6 +328,47 @@ int ensure_buffers(cfg_batch* b) {
     return CFG_OK;
 }
 
+// Parallel branches of a graph in capture on one stream, work going to them in turn.  The
+// stream's capture dependencies are set from branch to branch, so it takes no other stream
+// (about 50 us each) and no event.
+struct Branches {
+    static constexpr uint32_t N = 4;
+    std::vector<cudaGraphNode_t> tail[N];
+    uint32_t at = 0;
+    cudaError_t save(cudaStream_t s, std::vector<cudaGraphNode_t>& to) {   // what the stream depends on now
+        cudaStreamCaptureStatus st = cudaStreamCaptureStatusNone;
+        const cudaGraphNode_t* deps = nullptr;
+        size_t n = 0;
+        const cudaError_t e = cudaStreamGetCaptureInfo_v2(s, &st, nullptr, nullptr, &deps, &n);
+        if (e != cudaSuccess) return e;
+        if (st != cudaStreamCaptureStatusActive) return cudaErrorStreamCaptureInvalidated;
+        to.assign(deps, deps + n);
+        return cudaSuccess;
+    }
+    cudaError_t set(cudaStream_t s, std::vector<cudaGraphNode_t>& to) {
+        return cudaStreamUpdateCaptureDependencies(s, to.data(), to.size(), cudaStreamSetCaptureDependencies);
+    }
+    cudaError_t fork(cudaStream_t s) {
+        const cudaError_t e = save(s, tail[0]);
+        for (uint32_t q = 1; q < N; ++q) tail[q] = tail[0];
+        at = N;   // none entered yet
+        return e;
+    }
+    cudaError_t next(cudaStream_t s) {   // to the next branch
+        const cudaError_t e = at < N ? save(s, tail[at]) : cudaSuccess;
+        at = at + 1 < N ? at + 1 : 0;
+        return e != cudaSuccess ? e : set(s, tail[at]);
+    }
+    cudaError_t join(cudaStream_t s) {
+        const cudaError_t e = at < N ? save(s, tail[at]) : cudaSuccess;
+        std::vector<cudaGraphNode_t> all;
+        for (const auto& t : tail)
+            for (cudaGraphNode_t x : t)
+                if (std::find(all.begin(), all.end(), x) == all.end()) all.push_back(x);
+        return e != cudaSuccess ? e : set(s, all);
+    }
+};
+
 // The device work of one run, in stream order (captured into the graph).
 int enqueue(cfg_batch* b) {
     cudaStream_t s = b->stream;
@@ -399,20 +437,16 @@ int enqueue(cfg_batch* b) {
     // the classes, largest tables first, on four branches in turn: a class's last CTAs leave SMs
     // idle that the next class's can use (40 genomes of 0.5 to 8 Mbp: 29.7 -> 28.7 ms a call, 26 of
     // 0.4 to 3.5: 11.9 -> 11.4)
-    BCK(cudaEventRecord(b->fork_ev, s));
-    for (int q = 0; q < cfg_batch::SIDES; ++q) BCK(cudaStreamWaitEvent(b->side[q], b->fork_ev, 0));
-    uint32_t turn = 0;
+    Branches branches;
+    BCK(branches.fork(s));
     for (auto sh = b->shapes.rbegin(); sh != b->shapes.rend(); ++sh) {
-        const uint32_t q = turn++ % (cfg_batch::SIDES + 1);
         a.list_base = &bw->off[sh->cls];
         a.list_n = &bw->count[sh->cls];
-        BCK(launch_subgraphs_persistent(a, b->words, sh->cluster, sh->threads, sh->per, sh->grid, q ? b->side[q - 1] : s));
+        BCK(branches.next(s));
+        BCK(launch_subgraphs_persistent(a, b->words, sh->cluster, sh->threads, sh->per, sh->grid, s));
         ++launches;
     }
-    for (int q = 0; q < cfg_batch::SIDES; ++q) {
-        BCK(cudaEventRecord(b->join_ev[q], b->side[q]));
-        BCK(cudaStreamWaitEvent(s, b->join_ev[q], 0));
-    }
+    BCK(branches.join(s));
     k_job_finalize<<<b->n_jobs, 256, 0, s>>>(b->bucket_cnt.as<uint32_t>(), b->g_shift, b->jobs.as<JobOut>(),
                                              b->job_cur.as<unsigned long long>());
     ++launches;
@@ -529,10 +563,6 @@ int cfg_batch_create(int device, const cfg_params* params, cfg_batch** out) {
     if (cudaStreamCreateWithFlags(&b->stream, cudaStreamNonBlocking) != cudaSuccess) { delete b; return CFG_ERR_CUDA; }
     for (auto& e : b->ev)
         if (cudaEventCreate(&e) != cudaSuccess) { cfg_batch_destroy(b); return CFG_ERR_CUDA; }
-    if (cudaEventCreateWithFlags(&b->fork_ev, cudaEventDisableTiming) != cudaSuccess) { cfg_batch_destroy(b); return CFG_ERR_CUDA; }
-    for (int q = 0; q < cfg_batch::SIDES; ++q)
-        if (cudaStreamCreateWithFlags(&b->side[q], cudaStreamNonBlocking) != cudaSuccess ||
-            cudaEventCreateWithFlags(&b->join_ev[q], cudaEventDisableTiming) != cudaSuccess) { cfg_batch_destroy(b); return CFG_ERR_CUDA; }
     *out = b;
     return CFG_OK;
 }
@@ -975,9 +1005,6 @@ void cfg_batch_destroy(cfg_batch* b) {
     for (DevBuf* x : ubufs) x->release();
     if (b->plain) cfg_destroy(b->plain);
     for (auto& e : b->ev) if (e) cudaEventDestroy(e);
-    if (b->fork_ev) cudaEventDestroy(b->fork_ev);
-    for (auto& e : b->join_ev) if (e) cudaEventDestroy(e);
-    for (auto& x : b->side) if (x) cudaStreamDestroy(x);
     if (b->stream) cudaStreamDestroy(b->stream);
     delete b;
 }

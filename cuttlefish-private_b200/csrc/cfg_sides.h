@@ -15,14 +15,8 @@ class SideStreams {
 public:
     static constexpr uint32_t N = 3;
 
-    cudaError_t create() {
-        cudaError_t e = cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming);
-        for (uint32_t q = 0; q < N && e == cudaSuccess; ++q) {
-            e = cudaStreamCreateWithFlags(&side_[q], cudaStreamNonBlocking);
-            if (e == cudaSuccess) e = cudaEventCreateWithFlags(&join_[q], cudaEventDisableTiming);
-        }
-        return e;
-    }
+    // (a stream is made when a pass first has a launch for it: about 50 us each, an event 1 us)
+    cudaError_t create() { return cudaEventCreateWithFlags(&fork_, cudaEventDisableTiming); }
     void destroy() {
         for (uint32_t q = 0; q < N; ++q) {
             if (side_[q]) { cudaStreamSynchronize(side_[q]); cudaStreamDestroy(side_[q]); }
@@ -39,9 +33,12 @@ public:
     }
     cudaError_t on(cudaStream_t main, uint32_t t, cudaStream_t& out) {
         const uint32_t q = t % (N + 1);
+        cudaError_t e = cudaSuccess;
+        if (q && !side_[q - 1]) e = cudaStreamCreateWithFlags(&side_[q - 1], cudaStreamNonBlocking);
+        if (q && !join_[q - 1] && e == cudaSuccess) e = cudaEventCreateWithFlags(&join_[q - 1], cudaEventDisableTiming);
         out = q ? side_[q - 1] : main;
-        if (!q || (used_ >> q & 1)) return cudaSuccess;
-        const cudaError_t e = cudaStreamWaitEvent(out, fork_, 0);
+        if (!q || (used_ >> q & 1) || e != cudaSuccess) return e;
+        e = cudaStreamWaitEvent(out, fork_, 0);
         if (e == cudaSuccess) used_ |= 1u << q;
         return e;
     }

@@ -14,6 +14,7 @@ enum Kind { LAUNCH, RECORD, WAIT, SYNC };
 struct Op { Kind kind; const void* stream; const void* event; };
 std::vector<Op> g_ops;
 long g_calls = 0, g_fail_at = -1;   // calls that may fail so far; the one that does
+long g_streams = 0;                 // made so far
 uintptr_t g_next = 0x1000;
 
 size_t g_room = SIZE_MAX, g_asked = 0;   // device bytes left to give out; bytes given out since the last reset
@@ -27,7 +28,7 @@ extern "C" {
 
 cudaError_t cudaStreamCreateWithFlags(cudaStream_t* s, unsigned) {
     const cudaError_t e = step();
-    if (e == cudaSuccess) *s = (cudaStream_t)(g_next += 16);
+    if (e == cudaSuccess) { *s = (cudaStream_t)(g_next += 16); ++g_streams; }
     return e;
 }
 cudaError_t cudaStreamDestroy(cudaStream_t) { return cudaSuccess; }
@@ -90,6 +91,23 @@ uint64_t parse_state_bytes(uint64_t bytes) {
     const bool ok = pb.ensure_chunks((bytes + 4095) / 4096 + 1);
     pb.release();
     return ok ? g_asked : 0;
+}
+
+// Streams made by a SideStreams for a first pass of `launches` launches and a second one.
+int side_streams_made(uint32_t launches) {
+    cfg::SideStreams s;
+    g_fail_at = -1;
+    g_streams = 0;
+    bool ok = s.create() == cudaSuccess && g_streams == 0;
+    const cudaStream_t main_stream = (cudaStream_t)(g_next += 16);
+    for (int pass = 0; pass < 2; ++pass) {
+        ok = ok && s.fork(main_stream) == cudaSuccess;
+        cudaStream_t on = nullptr;
+        for (uint32_t t = 0; t < launches; ++t) ok = ok && s.on(main_stream, t, on) == cudaSuccess && on;
+        ok = ok && s.join(main_stream, false) == cudaSuccess;
+    }
+    s.destroy();
+    return ok ? (int)g_streams : -1;
 }
 
 // One pass of `launches` launches in which call number fail_at fails (-1: none; the calls

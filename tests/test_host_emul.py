@@ -46,6 +46,12 @@ def test_side_streams_leave_nothing_running(emul, launches):
         assert emul.side_streams_pass(launches, at, ctypes.byref(ctypes.c_long())) == 0, f"call {at} of {calls.value}"
 
 
+@pytest.mark.parametrize("launches", [0, 1, 2, 3, 4, 9])
+def test_side_streams_are_made_when_used(emul, launches):
+    """A context, or a run with one table class, pays for no stream; every one is made once."""
+    assert emul.side_streams_made(launches) == min(3, max(0, launches - 1))
+
+
 @pytest.mark.parametrize("k", [31, 63, 65, 127])
 @pytest.mark.parametrize("n", [0, 1, 1000, 1 << 20])
 def test_collation_buffers_know_what_they_hold(emul, n, k):
