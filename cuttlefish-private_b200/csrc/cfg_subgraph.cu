@@ -1423,9 +1423,14 @@ constexpr LocalShape SHAPES_4[] = {{64, 64}, {128, 64}, {256, 64}, {560, 64}, {1
 
 // The kernels' shared-memory limit is always raised to the largest table any launch
 // uses (it is process-wide state: lowering it would break launches recorded in graphs).
+template <size_t N> constexpr uint32_t max_slots(const LocalShape (&shapes)[N]) { return shapes[N - 1].slots; }
 template <int W> constexpr size_t max_table_bytes() {
-    return (size_t)(W == 1 ? 8192 : W == 2 ? 7200 : 4816) * slot_bytes(W);
+    return (size_t)(W == 1 ? max_slots(SHAPES_1) : W == 2 ? max_slots(SHAPES_2) : max_slots(SHAPES_4)) * slot_bytes(W);
 }
+constexpr size_t SMEM_PER_CTA = 227 * 1024;
+static_assert(max_table_bytes<1>() + sizeof(Block) <= SMEM_PER_CTA && max_table_bytes<2>() + sizeof(Block) <= SMEM_PER_CTA &&
+              max_table_bytes<3>() + sizeof(Block) <= SMEM_PER_CTA && max_table_bytes<4>() + sizeof(Block) <= SMEM_PER_CTA,
+              "the largest table and its bookkeeping fit one CTA's shared memory");
 template <typename K>
 cudaError_t raise_smem_limit(K kernel, size_t bytes) {
     return cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, (int)bytes);
