@@ -9,8 +9,9 @@
 //   partition (every job's fragments; job j's subgraph g is bucket j*G + g)
 //   -> multi-block scan of the J*G buckets -> scatter
 //   -> classify every bucket into a table class by its instance count
-//      (one CTA with 64..4096 slots, a cluster of 2..8 CTAs, or a global-memory
-//      table carved from an arena with a device-side bump allocator)
+//      (one CTA with 64..8192 slots, 64..4096 for k > 32, a cluster of 3..8 CTAs for
+//      k <= 31, or a global-memory table carved from an arena with a device-side bump
+//      allocator)
 //   -> give every job output regions sized from its record and instance counts
 //   -> one persistent launch per class, striding through that class's list, the
 //      classes on parallel branches.

@@ -322,8 +322,9 @@ uint64_t bucket_sort_scratch_words(uint32_t G, uint32_t sms) {
 cudaError_t launch_bucket_sort(const uint64_t* flat, const unsigned long long* n_dev, uint64_t cap, uint64_t n_bases, uint32_t G, uint32_t k, uint32_t sms, uint32_t* scratch,
                                uint64_t* tmp, uint64_t* out, uint32_t* bucket_off, uint32_t* inst, cudaStream_t s) {
     const uint32_t gbits = 31 - __builtin_clz(G), hbits = gbits < 10 ? gbits : 10, lbits = gbits - hbits;
-    // slabs: one CTA of k_sb_move_hi per SM, but some 2048 records each at least (6 bases a
-    // record): the (super-bucket, slab) counts of a 50 kbp job are then 5 k, not 151 k, to scan
+    // slabs: one CTA of k_sb_move_hi per SM, but 12288 bases each at least, some 2048 records at
+    // k = 31, l = 20 (2 / (k - l + 1) of them a base: 560 at k = 63, 230 at k = 127): the
+    // (super-bucket, slab) counts of a 50 kbp job are then 5 k, not 151 k, to scan
     const uint64_t slabs = n_bases / (6 * 2048) + 1;
     const uint32_t H = 1u << hbits, S = (uint32_t)(slabs < sms ? slabs : sms);
     const uint64_t m = (uint64_t)H * S;

@@ -11,7 +11,8 @@
 //      list's head and the label bases before it (each lm-tig adds its length minus
 //      the k-base overlap).  Sparse ruling set (Reid-Miller's list ranking; the GPU
 //      form of Rehman, Kothapalli & Narayanan, ICS 2009): heads, tails and a hashed
-//      1/16 sample of the entries are splitters; from every splitter one thread walks
+//      sample of the entries (a sixteenth; a quarter of sets under 500,000 lm-tigs)
+//      are splitters; from every splitter one thread walks
 //      back to the previous splitter, labelling the entries it passes with their
 //      distance to it; pointer jumping then ranks the splitters alone, and one pass
 //      gives every entry its rank from its splitter's;

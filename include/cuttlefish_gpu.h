@@ -67,8 +67,8 @@ typedef struct cfg_params {
                                  rebuild of the tables that overflow. */
     uint32_t slots_per_thread; /* one-CTA subgraph tables run slots / slots_per_thread threads (rounded
                                   up to whole warps, at least 64, at most the kernel form's largest
-                                  CTA); 0 = chosen with the table's size.  Speed only: results never
-                                  depend on it. */
+                                  CTA, which tables of more than 4096 slots always run); 0 = chosen
+                                  with the table's size.  Speed only: results never depend on it. */
     uint32_t reserved;
 } cfg_params;
 
